@@ -99,9 +99,14 @@ struct foggy_handle_s {
     double* d_rj = nullptr;
     double* d_delta = nullptr;    // d^j(pi/2), build_delta_table
     float* d_delta32 = nullptr;   // the same in single precision
+    double* d_frag = nullptr;     // the tensor-core operator's tables (build_mma_tables)
+    double* d_wf = nullptr;
+    int* d_plan = nullptr;
     int K = 0;
     // operator launches: (target bucket, source bucket) pairs of truncation-order buckets
     std::vector<DirectBucket> launches_direct;
+    std::vector<DirectBucket> launches_mma;   // the same launches with the tensor-core operator's chunks
+    int* d_slabs_used = nullptr;              // [target bucket][source bucket] its chunks, then each sphere's bucket
     int* d_bucket_lists = nullptr;
     int nbuckets = 0, cmax = 1;
     // waves and right-hand side
@@ -376,6 +381,8 @@ struct OrderTables {
     std::vector<int64_t> koffS;
     std::vector<double> gs, sb, rs, irs, rj, delta, g;
     std::vector<float> delta32;
+    std::vector<double> frag, wf;   // the tensor-core operator's tables
+    std::vector<int> plan;
 };
 
 std::shared_ptr<const OrderTables> order_tables(int pmax) {
@@ -412,6 +419,7 @@ std::shared_ptr<const OrderTables> order_tables(int pmax) {
     build_delta_table(pmax, t->delta);
     t->delta32.assign(t->delta.begin(), t->delta.end());
     build_g_table(pmax, t->g);
+    build_mma_tables(pmax, t->delta, t->frag, t->wf, t->plan);
     cache[pmax] = t;
     return t;
 }
@@ -419,9 +427,12 @@ std::shared_ptr<const OrderTables> order_tables(int pmax) {
 // the operator's order tables for degrees <= pmax on the device
 int ensure_tables(foggy_handle h, int pmax) {
     if (h->tab_pmax >= pmax) return FOGGY_OK;
-    for (double** q : {&h->d_gs, &h->d_sqrt_binom, &h->d_rs, &h->d_irs, &h->d_rj, &h->d_g, &h->d_delta}) dfree(h, *q);
+    for (double** q : {&h->d_gs, &h->d_sqrt_binom, &h->d_rs, &h->d_irs, &h->d_rj, &h->d_g, &h->d_delta, &h->d_frag,
+                       &h->d_wf})
+        dfree(h, *q);
     dfree(h, h->d_koffS);
     dfree(h, h->d_delta32);
+    dfree(h, h->d_plan);
     const std::shared_ptr<const OrderTables> t = order_tables(pmax);
     auto up = [&](auto** d, const auto& v) -> int {
         TRY(dalloc(h, d, v.size()));
@@ -437,6 +448,9 @@ int ensure_tables(foggy_handle h, int pmax) {
     TRY(up(&h->d_delta, t->delta));
     TRY(up(&h->d_delta32, t->delta32));
     TRY(up(&h->d_g, t->g));
+    TRY(up(&h->d_frag, t->frag));
+    TRY(up(&h->d_wf, t->wf));
+    TRY(up(&h->d_plan, t->plan));
     // the cached host vectors outlive the copies (the cache keeps them), so no synchronisation here
     h->gs_nm = pmax + 1;
     h->K = t->K;
@@ -481,6 +495,16 @@ DTabs dtabs(foggy_handle h) {
     t.K = h->K;
     return t;
 }
+
+MmaTabs mma_tabs(foggy_handle h) {
+    return MmaTabs{reinterpret_cast<const double2*>(h->d_frag), reinterpret_cast<const double2*>(h->d_wf),
+                   h->d_plan, h->tab_pmax + 8};
+}
+
+// Whether the FP64 operator runs on the tensor cores: over the pair tables, orders up to kMmaDegree.  It is the
+// faster one at every order it takes (222 spheres of one order: 7 0.29 against 1.39 ms, 15 0.76 / 2.0, 23 1.83 / 4.9,
+// 31 3.7 / 9.7); without tables k_direct's seven stages sum S where they use it.
+bool mma_operator(foggy_handle h, const DirectArgs& a) { return a.pt.stab && h->pmax <= kMmaDegree; }
 
 DirectArgs direct_args(foggy_handle h, const cplx* x) {
     DirectArgs a;
@@ -559,6 +583,33 @@ int plan_direct(foggy_handle h) {
             b.pp = std::max(bp[t], bp[s]);
             h->launches_direct.push_back(b);
         }
+    // The tensor-core operator takes the chunk count whose waves of CTAs cost least: a wave lasts as long as its
+    // CTAs' batches plus their set-up, about 0.3 of a batch.  64 spheres of order 15 (one wave of 256 CTAs with
+    // four batches each, where 14 chunks ran four waves of one batch): 109 -> 102 us an application; 1000 lognormal
+    // spheres: 29.9 -> 27.3 ms.
+    h->launches_mma = h->launches_direct;
+    std::vector<int> used;
+    for (DirectBucket& b : h->launches_mma) {
+        const int nb = (b.nsources + 3) / 4;
+        const int slots = 148 * mma_ctas_per_sm(b.pp);
+        double best = 1e300;
+        for (int c = 1; c <= std::min(nb, h->cmax); ++c) {
+            const double waves = std::ceil((double)b.ntargets * c / slots);
+            const double cost = waves * ((nb + c - 1) / c + 0.3);
+            if (cost < best * 0.999) {
+                best = cost;
+                b.chunks = c;
+            }
+        }
+        used.push_back(b.chunks);
+    }
+    const size_t first = used.size();
+    used.resize(first + h->N);
+    for (int t = 0; t < h->nbuckets; ++t)
+        for (int j : members[t]) used[first + j] = t;
+    dfree(h, h->d_slabs_used);
+    TRY(dalloc(h, &h->d_slabs_used, used.size()));
+    CK(h, h2d(h, h->d_slabs_used, used.data(), used.size() * sizeof(int)));
     return FOGGY_OK;
 }
 
@@ -1260,7 +1311,7 @@ int apply_operator_fmm(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false
     cudaEventRecord(h->ev_join, h->side);
     cudaStreamWaitEvent(h->stream, h->ev_join, 0);
     CKL(h);
-    k_direct_finish<<<h->N, 256, 0, h->stream>>>(sv, x, h->d_fmm_slab, 2, h->n_unk, y);
+    k_direct_finish<<<h->N, 256, 0, h->stream>>>(sv, x, h->d_fmm_slab, 2, 0, nullptr, h->n_unk, y);
     h->launches += 1;
     CKL(h);
     return FOGGY_OK;
@@ -1274,12 +1325,15 @@ int apply_operator(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false) {
     DirectArgs a = direct_args(h, x);
     a.fp32 = (fp32 && h->stab32_ready) ? 1 : 0;
     Trace tr(a.fp32 ? "operator (FP32)" : "operator (FP64)");
-    for (const DirectBucket& b : h->launches_direct) {
-        launch_direct(a, b, h->stream);
+    const bool mma = !a.fp32 && mma_operator(h, a);
+    for (const DirectBucket& b : mma ? h->launches_mma : h->launches_direct) {
+        if (mma) launch_direct_mma(a, mma_tabs(h), b, h->stream);
+        else launch_direct(a, b, h->stream);
         h->launches += 1;
     }
     CKL(h);
-    k_direct_finish<<<h->N, 256, 0, h->stream>>>(a.sc, x, h->d_partial, h->nbuckets * h->cmax, h->n_unk, y);
+    k_direct_finish<<<h->N, 256, 0, h->stream>>>(a.sc, x, h->d_partial, mma ? h->cmax : h->nbuckets * h->cmax,
+                                                 mma ? h->nbuckets : 0, h->d_slabs_used, h->n_unk, y);
     h->launches += 1;
     CKL(h);
     return FOGGY_OK;
@@ -1351,6 +1405,7 @@ void free_scene(foggy_handle h) {
     dfree(h, h->d_b);
     dfree(h, h->d_pq);
     dfree(h, h->d_partial);
+    dfree(h, h->d_slabs_used);
     dfree(h, h->d_stab);
     dfree(h, h->d_stab32);
     h->stab32_ready = false;
@@ -2572,10 +2627,11 @@ extern "C" int32_t foggy_matvec_static(foggy_handle h, const double* x, double* 
         DirectBucket b1 = b;
         b1.chunks = 1;
         b1.slab = b.slab / h->cmax;
-        launch_direct(a, b1, h->stream);
+        if (mma_operator(h, a)) launch_direct_mma(a, mma_tabs(h), b1, h->stream);
+        else launch_direct(a, b1, h->stream);
     }
     CKL(h);
-    k_direct_finish<<<h->N, 256, 0, h->stream>>>(sv, xin, partial, h->nbuckets, h->n_unk, yout);
+    k_direct_finish<<<h->N, 256, 0, h->stream>>>(sv, xin, partial, h->nbuckets, 0, nullptr, h->n_unk, yout);
     k_pack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, yout, xr, reinterpret_cast<cplx*>(y));
     CKL(h);
     CK(h, cudaStreamSynchronize(h->stream));

@@ -131,6 +131,21 @@ bool launch_direct_block(const BlockArgs& a, const DirectBucket& b, int R, cudaS
 size_t translation_pair_smem_bytes(int pmax);
 void launch_direct(const DirectArgs& a, const DirectBucket& b, cudaStream_t s);
 
+// k_direct_mma.cu -- the FP64 operator on the tensor cores, for orders up to kMmaDegree over the pair tables
+constexpr int kMmaDegree = 31;
+struct MmaTabs {
+    const double2* frag;       // d^n(pi/2) as fragments, degree by degree (build_mma_tables)
+    const double2* wf;         // factors of the coaxial step's w, one entry per (order, degree)
+    const int* plan;           // shared-memory layouts and warps' degrees by largest degree
+    int ld;                    // degrees per order of wf
+};
+void build_mma_tables(int pmax, const std::vector<double>& delta, std::vector<double>& frag, std::vector<double>& wf,
+                      std::vector<int>& plan);
+// CTAs of a launch of largest degree pp that an SM holds at once
+int mma_ctas_per_sm(int pp);
+// b.pp <= kMmaDegree, a.pt.stab set; fills slabs b.slab .. b.slab + b.chunks - 1
+void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, cudaStream_t s);
+
 // k_pair_tables.cu -- the pair tables over groups of pairs with one M2 = max order + 2: FP32 as
 // tensor-core products (tcgen05 kind::tf32, 3xTF32; the group's pairs share the Gaunt operand, a
 // tile is up to np pairs), FP64 summed on the CUDA cores (tiles of up to kPairs64 pairs).
@@ -173,9 +188,11 @@ struct PairArgs {
 };
 size_t pair_s_group_smem_bytes(int M2);
 void launch_pair_s_group(const PairArgs& a, int tile0, int ntiles, int M2, cudaStream_t s);
-// y = x + T (sum of the slab partials) for coupled spheres, y = x otherwise
-__global__ void k_direct_finish(SceneView sc, const cplx* x, const cplx* partial, int slabs, int64_t n_unk,
-                                cplx* y);
+// y = x + T (sum of the slab partials) for coupled spheres, y = x otherwise.  nbuckets = 0: all of `slabs` slabs;
+// otherwise `slabs` per source bucket, of which a target's bucket t fills used[t nbuckets + s], and sphere j's
+// bucket is used[nbuckets^2 + j]
+__global__ void k_direct_finish(SceneView sc, const cplx* x, const cplx* partial, int slabs, int nbuckets,
+                                const int* used, int64_t n_unk, cplx* y);
 // Sphere or box centres with their truncation orders and the offsets of their coefficient
 // vectors (scaled basis, a then b, standard (n, m) order).
 struct PointSet {

@@ -1,0 +1,186 @@
+// The FP64 direct operator on the tensor cores (k_mma.cuh): one CTA per target sphere and chunk of a
+// source bucket, four sources per batch.  Same launches, slabs and result layout as k_direct.
+#include <cmath>
+
+#include "k_mma.cuh"
+
+namespace foggy {
+
+namespace {
+using namespace mma;
+
+// direction of the translation from source l to target j, t = k (d_l - d_j), rounded as in disp_vec
+__device__ inline Dir pair_dir(const SceneView& sc, int j, int l) {
+    const double* ct = sc.centres + 3 * (size_t)j;
+    const double* cs = sc.centres + 3 * (size_t)l;
+    const double d0 = __dmul_rn(sc.k, __dsub_rn(cs[0], ct[0]));
+    const double d1 = __dmul_rn(sc.k, __dsub_rn(cs[1], ct[1]));
+    const double d2 = __dmul_rn(sc.k, __dsub_rn(cs[2], ct[2]));
+    return direction(d0, d1, d2, sqrt(__fma_rn(d0, d0, __fma_rn(d1, d1, __dmul_rn(d2, d2)))));
+}
+
+// records are made once in eight batches: a call keeps their arithmetic out of the loop's code
+__device__ __noinline__ Dir pair_dir_call(const SceneView& sc, int j, int l) { return pair_dir(sc, j, l); }
+}  // namespace
+
+template <int NI, int W, int CTAS>
+__global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTabs mt, DirectBucket bk, int us) {
+    extern __shared__ __align__(16) double smem_d[];
+    const SceneView& sc = a.sc;
+    const int j = bk.targets[blockIdx.x];
+    if (!sc.couple[j]) return;
+    constexpr int T = 32 * W, LD = phase_ld<NI>();
+    const int pp = bk.pp, c = blockIdx.y;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Shared s = carve<NI>(smem_d, pp, us);
+    const int pj = sc.p[j], Pj = pj * (pj + 2);
+    const int nb = (bk.nsources + kUnits - 1) / kUnits;   // batches of the bucket; this CTA: c, c + chunks, ...
+
+    // records of this CTA's batches 8g..8g+7, one unit per lane (one warp)
+    auto records = [&](int g) {
+        const int b = c + (8 * g + lane / kUnits) * bk.chunks, i = kUnits * b + lane % kUnits;
+        const int l = (b < nb && i < bk.nsources) ? bk.sources[i] : j;
+        Dir d{1.0, 0.0, 1.0, 0.0, 1.0};
+        Unit un{nullptr, nullptr, 0, -1, 1.0};
+        if (l != j) {
+            un.x = reinterpret_cast<const double2*>(a.x + sc.off[l]);
+            un.s = reinterpret_cast<const double2*>(a.pt.stab + a.pt.pair_off[pair_index(min(j, l), max(j, l), sc.n)]);
+            un.p = sc.p[l];
+            d = pair_dir_call(sc, j, l);
+            un.rho = d.rho;
+            un.km = d.rho == 0.0 ? -1 : min(pj, un.p);
+        }
+        s.dir[(g & 1) * kRecs + lane] = d;
+        s.un[(g & 1) * kRecs + lane] = un;
+    };
+    auto slot = [](int i) { return ((i >> 3) & 1) * kRecs + (i & 7) * kUnits; };   // records of batch i
+    // phase tables of batch i into half e; its coaxial rows are fetched into L2 meanwhile
+    auto prep = [&](int i, int e) {
+        const int at = slot(i);
+#pragma unroll 1
+        for (int t = tid; t < 2 * kUnits * LD; t += T) {
+            const int half = t / (kUnits * LD), r = t - half * kUnits * LD;
+            const int u = r / LD, m = r - u * LD;
+            const Dir& g = s.dir[at + u];
+            // e^{i m (phi + pi/2)}, or (-1)^s (2 cos s theta, 2 sin s theta) with (1, 0) at s = 0
+            const cplx z = zpow(half ? mk(g.ct, g.st) : mk(-g.sp, g.cp), m);
+            const double f = !half || m == 0 ? 1.0 : (m & 1) ? -2.0 : 2.0;
+            (half ? s.eth : s.eps)[e * kUnits * LD + r] = make_double2(f * z.x, f * z.y);
+        }
+        if (warp == W - 1) {
+#pragma unroll 1
+            for (int u = 0; u < kUnits; ++u) {
+                const Unit& un = s.un[at + u];
+                const int M2 = max(pj, un.p) + 2;
+                if (lane <= un.km) {
+                    // rows mu = k..pl + 1 of the order's square block: 16-byte entries, so aligned
+                    const unsigned bytes = (unsigned)((un.p + 2 - lane) * (M2 - lane) * sizeof(cplx));
+                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(un.s + block_offset(lane, M2)),
+                                 "r"(bytes)
+                                 : "memory");
+                }
+            }
+        }
+    };
+
+    for (int t = tid; t < kPlanInts; t += T) s.blk[t] = mt.plan[kPlanInts * pp + t];
+    if (tid < 4) s.zero[tid] = make_double2(0.0, 0.0);
+    for (int t = tid; t < 2 * Pj; t += T) s.acc[t] = make_double2(0.0, 0.0);
+    for (int t = tid; t < 8 * NI + 8; t += T) s.rn[t] = t ? 0.5 / (double)(t * (t + 1)) : 0.0;
+    if (warp == W - 1) records(0);
+    __syncthreads();
+    prep(0, 0);
+    const Lane<NI> L(s, pp, lane);
+    __syncthreads();
+    int cur = 0;
+    const int mine = c < nb ? (nb - c + bk.chunks - 1) / bk.chunks : 0;   // batches of this CTA
+    for (int ib = 0; ib < mine; ++ib, cur ^= 1) {
+        const Unit* un = s.un + slot(ib);
+        const int pl4 = max(max(un[0].p, un[1].p), max(un[2].p, un[3].p));
+        const Unit mine_u = un[L.u];   // this lane's unit in the rotations
+        // one copy of the rotation's code for both directions
+#pragma unroll 1
+        for (int out = 0; out < 2; ++out) {
+            rotate_all<NI>(s, L, mt.frag, warp, out ? pj : pl4, pj, mine_u, cur, out != 0);
+            if (out) break;
+            __syncthreads();
+            coaxial<NI>(s, un[warp % kUnits], warp % kUnits, warp / kUnits, W / kUnits, pj, mt.wf, mt.ld, lane);
+            if (ib + 1 < mine) {
+                prep(ib + 1, cur ^ 1);
+                // the next eight batches' records go where the last eight's were
+                if ((ib & 7) == 5 && warp == (ib >> 3) % W) records((ib >> 3) + 1);
+            }
+            __syncthreads();
+        }
+        if (un[0].rho == 0.0 || un[1].rho == 0.0 || un[2].rho == 0.0 || un[3].rho == 0.0) {
+            // coincident centres: the source is added unchanged, by the warp that owns the degree
+            __syncwarp();
+            for (int i = s.wfirst[warp]; i < s.wfirst[warp + 1]; ++i) {
+                const int n = s.ord[i];
+                for (int u = 0; u < kUnits; ++u)
+                    if (un[u].rho == 0.0 && n <= min(pj, un[u].p))
+                        for (int e = lane; e < 2 * (2 * n + 1); e += 32) {
+                            const int part = e > 2 * n, m = e - part * (2 * n + 1);
+                            const double2 v = un[u].x[part * un[u].p * (un[u].p + 2) + n * n - 1 + m];
+                            double2* d = s.acc + part * Pj + n * n - 1 + m;
+                            d->x += v.x;
+                            d->y += v.y;
+                        }
+            }
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    cplx* out = a.partial + (size_t)(bk.slab + c) * a.n_unk + sc.off[j];
+    for (int t = tid; t < 2 * Pj; t += T) out[t] = mk(s.acc[t].x, s.acc[t].y);
+}
+
+template <int NI, int W, int CTAS>
+static void launch_mma_t(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, cudaStream_t s) {
+    const size_t smem = mma::smem_bytes<NI>(b.pp);
+    raise_smem_ceiling(reinterpret_cast<const void*>(k_direct_mma<NI, W, CTAS>), smem);
+    k_direct_mma<NI, W, CTAS><<<dim3(b.ntargets, b.chunks), 32 * W, smem, s>>>(a, mt, b, mma::unit_size(b.pp));
+}
+
+int mma_ctas_per_sm(int pp) { return pp <= 7 ? 4 : pp <= 23 ? 2 : 1; }
+
+void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, cudaStream_t s) {
+    if (b.pp <= 7) launch_mma_t<1, mma::warps_of(7), 4>(a, mt, b, s);
+    else if (b.pp <= 15) launch_mma_t<2, mma::warps_of(15), 2>(a, mt, b, s);
+    else if (b.pp <= 23) launch_mma_t<3, mma::warps_of(23), 2>(a, mt, b, s);
+    else launch_mma_t<4, mma::warps_of(31), 1>(a, mt, b, s);
+}
+
+// The host tables of the tensor-core operator for degrees <= pmax (k_mma.cuh).
+void build_mma_tables(int pmax, const std::vector<double>& delta, std::vector<double>& frag, std::vector<double>& wf,
+                      std::vector<int>& plan) {
+    frag.clear();
+    for (int n = 1; n <= pmax; ++n) {
+        const double* Q = delta.data() + (size_t)n * (n + 1) * (2 * n + 1) / 6;
+        const int tiles = (mma::steps_of(n) + 1) / 2;
+        for (int P = 0; P < 2; ++P)
+            for (int t = 0; t < tiles; ++t)
+                for (int r = 0; r < 2; ++r)
+                    for (int jp = 0; jp < tiles; ++jp)
+                        for (int lane = 0; lane < 32; ++lane)
+                            for (int e = 0; e < 2; ++e) {
+                                const int c = lane >> 2;   // column: output order 8t + 4 (c & 1) + c / 2
+                                const int in = 2 * (4 * (2 * jp + e) + (lane & 3)) + r;
+                                const int out = 2 * (8 * t + 4 * (c & 1) + (c >> 1)) + P;
+                                frag.push_back(in <= n && out <= n ? Q[(size_t)in * (n + 1) + out] : 0.0);
+                            }
+    }
+    plan.assign((size_t)mma::kPlanInts * (kMmaDegree + 1), 0);
+    for (int pp = 1; pp <= kMmaDegree; ++pp) mma::make_plan(pp, mma::warps_of(pp), plan.data() + (size_t)mma::kPlanInts * pp);
+    // rows padded: the coaxial step reads whole k-steps of 4
+    const int ld = pmax + 8;
+    wf.assign(2 * (size_t)(pmax + 1) * ld, 0.0);
+    for (int k = 0; k <= pmax; ++k)
+        for (int mu = k; mu < ld; ++mu) {
+            double* f = wf.data() + 2 * ((size_t)k * ld + mu);
+            f[0] = 2.0 * (mu - 1.0) * std::sqrt((double)mu * mu - (double)k * k);
+            f[1] = 2.0 * (mu + 2.0) * std::sqrt((mu + 1.0) * (mu + 1.0) - (double)k * k);
+        }
+}
+
+}  // namespace foggy
