@@ -96,7 +96,10 @@ typedef struct foggy_params {
                                     coaxial blocks, rotations and coaxial sums; FP64 vectors
                                     and box coefficients), the true residual at the start and
                                     at every restart in FP64, so the restarts refine to
-                                    gmres_tolerance.  foggy_matvec stays FP64.               */
+                                    gmres_tolerance.  foggy_matvec stays FP64.  Where the
+                                    FP64 operator runs on the tensor cores (pair tables kept,
+                                    orders up to 31) it is as fast, and the Arnoldi steps of
+                                    the direct operator use it instead                      */
 } foggy_params;
 
 /* Per-solve statistics (the reference prints these; here they are returned). */
@@ -345,13 +348,15 @@ int32_t foggy_matvec_rhs(foggy_handle h, int32_t nrhs, const double* x, double* 
 /* The right-hand sides of one scene (one per plane wave set on the handle, nrhs = that count; no
  * Gaussian beams) solved together.  The reference solves each illumination with its own GMRES run
  * (lib_mie_ms_solver_run, lib_mie_ms_solver_interface.f90:143-154, around lib_solver_GMRES.f90:116-316);
- * here every operator application serves the whole block: each CTA of the operator applies the
+ * here every operator application serves the whole block: over the pair tables, orders up to 31, one
+ * right-hand side per CTA on the FP64 tensor cores; otherwise (and in FP32) each CTA applies the
  * translations of one target sphere to a tile of right-hand sides, whose width the library picks per
  * launch shape by timing (foggy_block_tiles); with matvec_mode = FOGGY_MATVEC_MLFMM the passes run
  * vector after vector inside each block application.  Each right-hand side keeps its own GMRES(m) recurrence
  * (gmres_restart 1..63, gmres_tolerance, gmres_max_iterations apply to each) and leaves the block when
  * its true residual meets the tolerance at a restart.  With params.precision = 1 the Arnoldi steps
- * apply the operator with FP32 translation arithmetic and the restart residuals in FP64.  x (and x0, if
+ * apply the operator with FP32 translation arithmetic (unless the FP64 tensor-core operator runs, see
+ * foggy_params.precision) and the restart residuals in FP64.  x (and x0, if
  * not NULL) hold nrhs vectors of foggy_vector_length entries one after the other; cross_sections
  * ({C_sca, C_ext, C_abs} per right-hand side), iterations and backward_errors (per right-hand side) may
  * be NULL.  stats: iterations summed over right-hand sides, matvecs = vectors the operator was applied
@@ -367,7 +372,7 @@ int32_t foggy_matvec_block(foggy_handle h, int32_t nrhs, int32_t precision, cons
 
 /* The block operator's tile width per launch for a block of nrhs vectors, tuned on first use:
  * out[4 i + 0..3] = (target spheres, source spheres, largest degree, right-hand sides per CTA) of
- * launch i.  out = NULL queries the launch count.  No counterpart in the reference. */
+ * launch i (1 per CTA, nothing to tune, where the FP64 tensor-core operator runs).  out = NULL queries the launch count.  No counterpart in the reference. */
 int32_t foggy_block_tiles(foggy_handle h, int32_t precision, int32_t nrhs, int32_t* out, int32_t* count);
 
 /* ---- serving ------------------------------------------------------------------------- */

@@ -43,6 +43,12 @@ struct Trace {
     Trace& operator=(const Trace&) = delete;
 };
 
+// The direct operator's launches with the tensor-core operator's chunks for a number of vectors, and the slabs they fill.
+struct MmaPlan {
+    std::vector<DirectBucket> launches;
+    SlabUse use{};
+};
+
 }  // namespace
 
 struct foggy_handle_s {
@@ -105,8 +111,7 @@ struct foggy_handle_s {
     int K = 0;
     // operator launches: (target bucket, source bucket) pairs of truncation-order buckets
     std::vector<DirectBucket> launches_direct;
-    std::vector<DirectBucket> launches_mma;   // the same launches with the tensor-core operator's chunks
-    int* d_slabs_used = nullptr;              // [target bucket][source bucket] its chunks, then each sphere's bucket
+    std::map<int, MmaPlan> mma_plans;   // the tensor-core operator's launches by number of vectors
     int* d_bucket_lists = nullptr;
     int nbuckets = 0, cmax = 1;
     // waves and right-hand side
@@ -583,34 +588,48 @@ int plan_direct(foggy_handle h) {
             b.pp = std::max(bp[t], bp[s]);
             h->launches_direct.push_back(b);
         }
-    // The tensor-core operator takes the chunk count whose waves of CTAs cost least: a wave lasts as long as its
-    // CTAs' batches plus their set-up, about 0.3 of a batch.  64 spheres of order 15 (one wave of 256 CTAs with
-    // four batches each, where 14 chunks ran four waves of one batch): 109 -> 102 us an application; 1000 lognormal
-    // spheres: 29.9 -> 27.3 ms.
-    h->launches_mma = h->launches_direct;
-    std::vector<int> used;
-    for (DirectBucket& b : h->launches_mma) {
-        const int nb = (b.nsources + 3) / 4;
-        const int slots = 148 * mma_ctas_per_sm(b.pp);
+    h->mma_plans.clear();
+    return FOGGY_OK;
+}
+
+// The tensor-core operator's launches for nrhs vectors at a time (at most h->cmax: each has its own slabs).  The
+// slabs of one vector and source bucket bound the chunks; among them the count is taken whose waves of CTAs cost
+// least: a wave lasts as long as its CTAs' batches plus their set-up, about 0.3 of a batch.  64 spheres of order 15
+// (one wave of 256 CTAs with four batches each, where 14 chunks ran four waves of one batch): 109 -> 102 us an
+// application; 1000 lognormal spheres: 29.9 -> 27.3 ms.
+const MmaPlan& mma_plan(foggy_handle h, int nrhs) {
+    auto it = h->mma_plans.find(nrhs);
+    if (it != h->mma_plans.end()) return it->second;
+    MmaPlan p;
+    p.launches = h->launches_direct;
+    const int nb = h->nbuckets, per = std::max(1, h->cmax / nrhs);
+    p.use.nb = nb;
+    p.use.per_bucket = per;
+    p.use.per_rhs = nb * per;
+    for (int i = 0; i < nb * nb; ++i) {
+        DirectBucket& b = p.launches[i];
+        const int t = i / nb, s = i % nb, batches = (b.nsources + 3) / 4;
+        const double slots = 148.0 * mma_ctas_per_sm(b.pp);
         double best = 1e300;
-        for (int c = 1; c <= std::min(nb, h->cmax); ++c) {
-            const double waves = std::ceil((double)b.ntargets * c / slots);
-            const double cost = waves * ((nb + c - 1) / c + 0.3);
+        for (int c = 1; c <= std::min(batches, per); ++c) {
+            const double cost = std::ceil((double)b.ntargets * nrhs * c / slots) * ((batches + c - 1) / c + 0.3);
             if (cost < best * 0.999) {
                 best = cost;
                 b.chunks = c;
             }
         }
-        used.push_back(b.chunks);
+        b.slab = s * per;
+        p.use.c[t][s] = (unsigned char)b.chunks;
     }
-    const size_t first = used.size();
-    used.resize(first + h->N);
-    for (int t = 0; t < h->nbuckets; ++t)
-        for (int j : members[t]) used[first + j] = t;
-    dfree(h, h->d_slabs_used);
-    TRY(dalloc(h, &h->d_slabs_used, used.size()));
-    CK(h, h2d(h, h->d_slabs_used, used.data(), used.size() * sizeof(int)));
-    return FOGGY_OK;
+    // compact bucket of each step of four orders
+    int id = 0;
+    for (int q = 0; q < 12; ++q) {
+        bool any = false;
+        for (int pj : h->p_s) any |= (pj - 1) / 4 == q;
+        p.use.of[q] = (unsigned char)id;
+        id += any;
+    }
+    return h->mma_plans.emplace(nrhs, std::move(p)).first->second;
 }
 
 // The pair tables over groups of pairs (k_pair_tables.cu).  The pairs are grouped by
@@ -726,7 +745,12 @@ int build_pair_tables(foggy_handle h, const SGaunt& g, bool fp64, bool fp32) {
 // and read by every operator application.  Skipped when they do not fit (pair_tables = 0) or
 // when switched off (pair_tables = -1).  The double-precision tables are FP64 sums on the CUDA
 // cores, the single-precision ones tensor-core products in 3xTF32 (build_pair_tables).
-int ensure_pair_tables(foggy_handle h) {
+// A mixed-precision handle's Arnoldi steps run the FP64 tensor-core operator where its orders and tables allow: it is as
+// fast as the FP32 one, and its solve needs no refinement cycles (250 lognormal spheres to 1e-11: 260 ms with FP32
+// steps, 148 with these; 32 right-hand sides of 64 spheres: 160 and 114).  So such a handle keeps the double-precision tables
+// alone where they fit, and the single-precision ones where they do not, above kMmaDegree, or where FP32 is asked for
+// by name (fp32).
+int ensure_pair_tables(foggy_handle h, bool fp32 = false) {
     const bool mixed = h->prm.precision == 1;
     if (h->prm.pair_tables < 0 || h->N < 2) {
         h->stab_ready = false;
@@ -739,7 +763,9 @@ int ensure_pair_tables(foggy_handle h) {
         h->stab_ready = false;
         h->stab32_ready = false;
     }
-    if (mixed ? h->stab32_ready : h->stab_ready) return FOGGY_OK;
+    const bool only64 = mixed && !fp32 && h->pmax <= kMmaDegree;
+    if ((!mixed || only64) && h->stab_ready) return FOGGY_OK;
+    if (mixed && h->stab32_ready) return FOGGY_OK;
     const int64_t npairs = (int64_t)h->N * (h->N - 1) / 2;
     // total size from the counts of each truncation order
     std::vector<int64_t> cnt(h->pmax + 1, 0);
@@ -760,13 +786,12 @@ int ensure_pair_tables(foggy_handle h) {
     const size_t room = h->budget > h->bytes_in_use ? h->budget - h->bytes_in_use : 0;
     const size_t reserve = (size_t)(h->prm.gmres_restart + 4) * (size_t)h->n_unk * sizeof(cplx) + ((size_t)4 << 30);
     const bool force = h->prm.pair_tables == 1;
-    const bool want32 = mixed && (force || offb + b32 + reserve <= room);
-    const bool want64 = mixed ? (force || offb + b32 + b64 + reserve <= room) : (force || offb + b64 + reserve <= room);
-    if (!want32 && !want64) {
-        h->stab_ready = false;
-        h->stab32_ready = false;
-        return FOGGY_OK;
-    }
+    const bool fits64 = force || offb + b64 + reserve <= room;
+    const bool want32 = mixed && !(only64 && fits64) && (force || offb + b32 + reserve <= room);
+    const bool want64 = want32 ? (force || offb + b32 + b64 + reserve <= room) : (!mixed || only64) && fits64;
+    // what is there stays (a precision that does not fit now takes nothing from the other)
+    const bool make32 = want32 && !h->stab32_ready, make64 = want64 && !h->stab_ready;
+    if (!make32 && !make64) return FOGGY_OK;
     if (!h->d_pair_off) {
         TRY(dalloc(h, &h->d_pair_off, npairs + 1));
         int64_t* d_sizes = nullptr;
@@ -786,11 +811,11 @@ int ensure_pair_tables(foggy_handle h) {
     }
     Trace tr("pair tables");
     SGaunt g{h->d_koffS, h->d_gs, h->gs_nm};
-    if (want64 && !h->d_stab) TRY(dalloc(h, &h->d_stab, (size_t)tot));
-    if (want32 && !h->d_stab32) TRY(dalloc(h, &h->d_stab32, (size_t)tot));
-    TRY(build_pair_tables(h, g, want64, want32));
-    if (want64) h->stab_ready = true;
-    if (want32) h->stab32_ready = true;
+    if (make64 && !h->d_stab) TRY(dalloc(h, &h->d_stab, (size_t)tot));
+    if (make32 && !h->d_stab32) TRY(dalloc(h, &h->d_stab32, (size_t)tot));
+    TRY(build_pair_tables(h, g, make64, make32));
+    if (make64) h->stab_ready = true;
+    if (make32) h->stab32_ready = true;
     CKL(h);
     h->stab_z = h->prm.z_coupling;
     return FOGGY_OK;
@@ -1311,10 +1336,21 @@ int apply_operator_fmm(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false
     cudaEventRecord(h->ev_join, h->side);
     cudaStreamWaitEvent(h->stream, h->ev_join, 0);
     CKL(h);
-    k_direct_finish<<<h->N, 256, 0, h->stream>>>(sv, x, h->d_fmm_slab, 2, 0, nullptr, h->n_unk, y);
+    SlabUse two{};
+    two.per_rhs = 2;
+    k_direct_finish<<<h->N, 256, 0, h->stream>>>(sv, x, h->d_fmm_slab, two, h->n_unk, 0, y);
     h->launches += 1;
     CKL(h);
     return FOGGY_OK;
+}
+
+// Y_r = A X_r on the tensor cores for the nrhs <= h->cmax vectors X + r n_unk
+void launch_mma(foggy_handle h, DirectArgs a, int nrhs, const cplx* X, cplx* Y) {
+    const MmaPlan& p = mma_plan(h, nrhs);
+    const MmaTabs mt = mma_tabs(h);
+    a.x = X;
+    for (const DirectBucket& b : p.launches) launch_direct_mma(a, mt, b, nrhs, h->n_unk, p.use.per_rhs, h->stream);
+    k_direct_finish<<<dim3(h->N, nrhs), 256, 0, h->stream>>>(a.sc, X, h->d_partial, p.use, h->n_unk, h->n_unk, Y);
 }
 
 // y = A x in the device layout
@@ -1323,18 +1359,19 @@ int apply_operator(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false) {
     if (h->prm.matvec_mode == FOGGY_MATVEC_MLFMM) return apply_operator_fmm(h, x, y, fp32);
     TRY(ensure_pair_tables(h));
     DirectArgs a = direct_args(h, x);
-    a.fp32 = (fp32 && h->stab32_ready) ? 1 : 0;
+    const bool mma = mma_operator(h, a);   // also for the Arnoldi steps of a mixed-precision solve
+    a.fp32 = (!mma && fp32 && h->stab32_ready) ? 1 : 0;
     Trace tr(a.fp32 ? "operator (FP32)" : "operator (FP64)");
-    const bool mma = !a.fp32 && mma_operator(h, a);
-    for (const DirectBucket& b : mma ? h->launches_mma : h->launches_direct) {
-        if (mma) launch_direct_mma(a, mma_tabs(h), b, h->stream);
-        else launch_direct(a, b, h->stream);
-        h->launches += 1;
+    if (mma) {
+        launch_mma(h, a, 1, x, y);
+    } else {
+        for (const DirectBucket& b : h->launches_direct) launch_direct(a, b, h->stream);
+        CKL(h);
+        SlabUse all{};
+        all.per_rhs = h->nbuckets * h->cmax;
+        k_direct_finish<<<h->N, 256, 0, h->stream>>>(a.sc, x, h->d_partial, all, h->n_unk, 0, y);
     }
-    CKL(h);
-    k_direct_finish<<<h->N, 256, 0, h->stream>>>(a.sc, x, h->d_partial, mma ? h->cmax : h->nbuckets * h->cmax,
-                                                 mma ? h->nbuckets : 0, h->d_slabs_used, h->n_unk, y);
-    h->launches += 1;
+    h->launches += (int64_t)h->launches_direct.size() + 1;
     CKL(h);
     return FOGGY_OK;
 }
@@ -1405,7 +1442,6 @@ void free_scene(foggy_handle h) {
     dfree(h, h->d_b);
     dfree(h, h->d_pq);
     dfree(h, h->d_partial);
-    dfree(h, h->d_slabs_used);
     dfree(h, h->d_stab);
     dfree(h, h->d_stab32);
     h->stab32_ready = false;
@@ -2627,11 +2663,13 @@ extern "C" int32_t foggy_matvec_static(foggy_handle h, const double* x, double* 
         DirectBucket b1 = b;
         b1.chunks = 1;
         b1.slab = b.slab / h->cmax;
-        if (mma_operator(h, a)) launch_direct_mma(a, mma_tabs(h), b1, h->stream);
+        if (mma_operator(h, a)) launch_direct_mma(a, mma_tabs(h), b1, 1, 0, h->nbuckets, h->stream);
         else launch_direct(a, b1, h->stream);
     }
     CKL(h);
-    k_direct_finish<<<h->N, 256, 0, h->stream>>>(sv, xin, partial, h->nbuckets, 0, nullptr, h->n_unk, yout);
+    SlabUse all{};
+    all.per_rhs = h->nbuckets;
+    k_direct_finish<<<h->N, 256, 0, h->stream>>>(sv, xin, partial, all, h->n_unk, 0, yout);
     k_pack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, yout, xr, reinterpret_cast<cplx*>(y));
     CKL(h);
     CK(h, cudaStreamSynchronize(h->stream));
@@ -2744,16 +2782,30 @@ BlockArgs block_args(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool fp32
     return ba;
 }
 
-// Y_r = A X_r for r < nrhs (device layout, n_unk apart), FP64 or FP32 translation arithmetic
-int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool fp32) {
+// Y_r = A X_r for r < nrhs (device layout, n_unk apart), FP64 or FP32 translation arithmetic; must32: FP32 was asked
+// for by name (otherwise the FP64 tensor-core operator stands in for it where it runs)
+int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool fp32, bool must32 = false) {
     if (h->prm.matvec_mode == FOGGY_MATVEC_MLFMM) {
         // the ML-FMM passes one vector after another (their translations are per box, not per pair)
         for (int r = 0; r < nrhs; ++r)
             TRY(apply_operator_fmm(h, X + (size_t)r * h->n_unk, Y + (size_t)r * h->n_unk, fp32));
         return FOGGY_OK;
     }
-    TRY(ensure_pair_tables(h));
+    TRY(ensure_pair_tables(h, must32));
     const BlockArgs ba = block_args(h, X, Y, nrhs, fp32);
+    if (!must32 && mma_operator(h, ba.d)) {
+        // as many vectors at a time as have slabs.  One vector per CTA: a batch's set-up that vectors could share is
+        // small beside its products, and the pair's coaxial block comes from L2 after the first.  83 spheres, 5
+        // right-hand sides to 1e-6: 161 -> 55 ms a request (the tile autotuner's runs are gone too)
+        Trace tr("block operator (FP64)");
+        for (int r = 0; r < nrhs; r += h->cmax) {
+            const int nr = std::min(h->cmax, nrhs - r);
+            launch_mma(h, ba.d, nr, X + (size_t)r * h->n_unk, Y + (size_t)r * h->n_unk);
+            h->launches += (int64_t)h->launches_direct.size() + 1;
+        }
+        CKL(h);
+        return FOGGY_OK;
+    }
     const bool tabs = fp32 ? ba.d.pt.stab32 != nullptr : ba.d.pt.stab != nullptr;
     Trace tr(fp32 ? "block operator (FP32)" : "block operator (FP64)");
     CK(h, cudaMemcpyAsync(Y, X, (size_t)nrhs * h->n_unk * sizeof(cplx), cudaMemcpyDeviceToDevice, h->stream));
@@ -3007,7 +3059,7 @@ int32_t foggy_matvec_block(foggy_handle h, int32_t nrhs, int32_t precision, cons
         }
         k_unpack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, src, X + (size_t)r * n);
     }
-    int rc = apply_operator_block(h, X, Y, nrhs, precision == 1);
+    int rc = apply_operator_block(h, X, Y, nrhs, precision == 1, precision == 1);
     if (rc) return fin(rc);
     for (int r = 0; r < nrhs; ++r) {
         const cplx* xr = reinterpret_cast<const cplx*>(x) + r * len;
@@ -3144,7 +3196,7 @@ int32_t foggy_block_tiles(foggy_handle h, int32_t precision, int32_t nrhs, int32
     CK(h, cudaSetDevice(h->device));
     *count = (int)h->launches_direct.size();
     if (!out) return FOGGY_OK;
-    TRY(ensure_pair_tables(h));
+    TRY(ensure_pair_tables(h, precision == 1));
     // the tuner reads the first min(nrhs, 16) vectors of the block: zeros serve
     cplx* X = nullptr;
     const int nrt = std::min(nrhs, 16);
@@ -3156,7 +3208,9 @@ int32_t foggy_block_tiles(foggy_handle h, int32_t precision, int32_t nrhs, int32
     for (size_t i = 0; i < h->launches_direct.size() && rc == FOGGY_OK; ++i) {
         const DirectBucket& b = h->launches_direct[i];
         int R = 0;
-        rc = choose_tile(h, ba, b, tabs, &R);
+        // one vector per CTA on the tensor cores
+        if (!ba.d.fp32 && mma_operator(h, ba.d)) R = 1;
+        else rc = choose_tile(h, ba, b, tabs, &R);
         out[4 * i] = b.ntargets;
         out[4 * i + 1] = b.nsources;
         out[4 * i + 2] = b.pp;

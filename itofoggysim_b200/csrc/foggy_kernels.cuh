@@ -143,8 +143,10 @@ void build_mma_tables(int pmax, const std::vector<double>& delta, std::vector<do
                       std::vector<int>& plan);
 // CTAs of a launch of largest degree pp that an SM holds at once
 int mma_ctas_per_sm(int pp);
-// b.pp <= kMmaDegree, a.pt.stab set; fills slabs b.slab .. b.slab + b.chunks - 1
-void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, cudaStream_t s);
+// b.pp <= kMmaDegree, a.pt.stab set; for each of nrhs vectors (a.x + r ld) fills slabs b.slab .. b.slab + b.chunks - 1
+// of the r-th run of per_rhs slabs
+void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, int nrhs, int64_t ld, int per_rhs,
+                       cudaStream_t s);
 
 // k_pair_tables.cu -- the pair tables over groups of pairs with one M2 = max order + 2: FP32 as
 // tensor-core products (tcgen05 kind::tf32, 3xTF32; the group's pairs share the Gaunt operand, a
@@ -188,11 +190,17 @@ struct PairArgs {
 };
 size_t pair_s_group_smem_bytes(int M2);
 void launch_pair_s_group(const PairArgs& a, int tile0, int ntiles, int M2, cudaStream_t s);
-// y = x + T (sum of the slab partials) for coupled spheres, y = x otherwise.  nbuckets = 0: all of `slabs` slabs;
-// otherwise `slabs` per source bucket, of which a target's bucket t fills used[t nbuckets + s], and sphere j's
-// bucket is used[nbuckets^2 + j]
-__global__ void k_direct_finish(SceneView sc, const cplx* x, const cplx* partial, int slabs, int nbuckets,
-                                const int* used, int64_t n_unk, cplx* y);
+// Which slabs a final sum reads: per right-hand side `per_rhs` slabs, source bucket s's from s per_bucket on; the
+// target's bucket of[(p - 1) / 4] fills c[bucket][s] of them.  nb = 0: the first per_rhs slabs, whatever the sphere.
+struct SlabUse {
+    int nb, per_rhs, per_bucket;
+    unsigned char of[12];
+    unsigned char c[12][12];
+};
+// y = x + T (sum of the slab partials) for coupled spheres, y = x otherwise; blockIdx.y = right-hand side (vectors
+// ld entries apart)
+__global__ void k_direct_finish(SceneView sc, const cplx* x, const cplx* partial, SlabUse use, int64_t n_unk, int64_t ld,
+                                cplx* y);
 // Sphere or box centres with their truncation orders and the offsets of their coefficient
 // vectors (scaled basis, a then b, standard (n, m) order).
 struct PointSet {

@@ -1470,22 +1470,25 @@ bool launch_direct_block(const BlockArgs& a, const DirectBucket& b, int R, cudaS
     return false;
 }
 
-// y = x + T (sum of the slabs) for coupled spheres, y = x otherwise.
-__global__ void k_direct_finish(SceneView sc, const cplx* x, const cplx* partial, int slabs, int nbuckets,
-                                const int* used, int64_t n_unk, cplx* y) {
+// y = x + T (sum of the slabs) for coupled spheres, y = x otherwise
+__global__ void k_direct_finish(SceneView sc, const cplx* x, const cplx* partial, SlabUse use, int64_t n_unk, int64_t ld,
+                                cplx* y) {
     int j = blockIdx.x;
     int pj = sc.p[j];
     int Pj = pj * (pj + 2);
     int64_t o = sc.off[j];
     bool cp = sc.couple[j] != 0;
-    const int* row = nbuckets ? used + nbuckets * used[nbuckets * nbuckets + j] : nullptr;
+    x += blockIdx.y * ld;
+    y += blockIdx.y * ld;
+    partial += (size_t)blockIdx.y * use.per_rhs * n_unk;
+    const int row = use.nb ? use.of[(pj - 1) >> 2] : 0;
     for (int t = threadIdx.x; t < 2 * Pj; t += blockDim.x) {
         cplx v = x[o + t];
         if (cp) {
             cplx sum = mk(0, 0);
-            for (int b = 0; b < (nbuckets ? nbuckets : 1); ++b) {
-                const cplx* q = partial + (size_t)b * slabs * n_unk + o + t;
-                const int m = row ? row[b] : slabs;
+            for (int b = 0; b < (use.nb ? use.nb : 1); ++b) {
+                const cplx* q = partial + (size_t)b * use.per_bucket * n_unk + o + t;
+                const int m = use.nb ? use.c[row][b] : use.per_rhs;
                 for (int c = 0; c < m; ++c) sum = sum + q[(size_t)c * n_unk];
             }
             int tt = t < Pj ? t : t - Pj;

@@ -24,11 +24,14 @@ __device__ __noinline__ Dir pair_dir_call(const SceneView& sc, int j, int l) { r
 }  // namespace
 
 template <int NI, int W, int CTAS>
-__global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTabs mt, DirectBucket bk, int us) {
+__global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTabs mt, DirectBucket bk, int us, int nrhs,
+                                                             int64_t ld, int per_rhs) {
     extern __shared__ __align__(16) double smem_d[];
     const SceneView& sc = a.sc;
-    const int j = bk.targets[blockIdx.x];
+    // right-hand side fastest: the CTAs that read one pair's coaxial block run together
+    const int rhs = blockIdx.x % nrhs, j = bk.targets[blockIdx.x / nrhs];
     if (!sc.couple[j]) return;
+    const cplx* const x = a.x + rhs * ld;
     constexpr int T = 32 * W, LD = phase_ld<NI>();
     const int pp = bk.pp, c = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -43,7 +46,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTa
         Dir d{1.0, 0.0, 1.0, 0.0, 1.0};
         Unit un{nullptr, nullptr, 0, -1, 1.0};
         if (l != j) {
-            un.x = reinterpret_cast<const double2*>(a.x + sc.off[l]);
+            un.x = reinterpret_cast<const double2*>(x + sc.off[l]);
             un.s = reinterpret_cast<const double2*>(a.pt.stab + a.pt.pair_off[pair_index(min(j, l), max(j, l), sc.n)]);
             un.p = sc.p[l];
             d = pair_dir_call(sc, j, l);
@@ -131,24 +134,23 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTa
         }
     }
     __syncthreads();
-    cplx* out = a.partial + (size_t)(bk.slab + c) * a.n_unk + sc.off[j];
+    cplx* out = a.partial + ((size_t)rhs * per_rhs + bk.slab + c) * a.n_unk + sc.off[j];
     for (int t = tid; t < 2 * Pj; t += T) out[t] = mk(s.acc[t].x, s.acc[t].y);
-}
-
-template <int NI, int W, int CTAS>
-static void launch_mma_t(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, cudaStream_t s) {
-    const size_t smem = mma::smem_bytes<NI>(b.pp);
-    raise_smem_ceiling(reinterpret_cast<const void*>(k_direct_mma<NI, W, CTAS>), smem);
-    k_direct_mma<NI, W, CTAS><<<dim3(b.ntargets, b.chunks), 32 * W, smem, s>>>(a, mt, b, mma::unit_size(b.pp));
 }
 
 int mma_ctas_per_sm(int pp) { return pp <= 7 ? 4 : pp <= 23 ? 2 : 1; }
 
-void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, cudaStream_t s) {
-    if (b.pp <= 7) launch_mma_t<1, mma::warps_of(7), 4>(a, mt, b, s);
-    else if (b.pp <= 15) launch_mma_t<2, mma::warps_of(15), 2>(a, mt, b, s);
-    else if (b.pp <= 23) launch_mma_t<3, mma::warps_of(23), 2>(a, mt, b, s);
-    else launch_mma_t<4, mma::warps_of(31), 1>(a, mt, b, s);
+void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, int nrhs, int64_t ld, int per_rhs,
+                       cudaStream_t s) {
+    auto go = [&](auto kernel, size_t smem) {
+        raise_smem_ceiling(reinterpret_cast<const void*>(kernel), smem);
+        kernel<<<dim3((unsigned)b.ntargets * nrhs, b.chunks), 32 * mma::warps_of(b.pp), smem, s>>>(
+            a, mt, b, mma::unit_size(b.pp), nrhs, ld, per_rhs);
+    };
+    if (b.pp <= 7) go(k_direct_mma<1, mma::warps_of(7), 4>, mma::smem_bytes<1>(b.pp));
+    else if (b.pp <= 15) go(k_direct_mma<2, mma::warps_of(15), 2>, mma::smem_bytes<2>(b.pp));
+    else if (b.pp <= 23) go(k_direct_mma<3, mma::warps_of(23), 2>, mma::smem_bytes<3>(b.pp));
+    else go(k_direct_mma<4, mma::warps_of(31), 1>, mma::smem_bytes<4>(b.pp));
 }
 
 // The host tables of the tensor-core operator for degrees <= pmax (k_mma.cuh).

@@ -92,3 +92,36 @@ def test_nan_stays_with_the_targets_it_reaches(native):
             y = s.calculate_vector_b(x)
         out.append(np.isnan(y.real) | np.isnan(y.imag))
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("nv", [1, 3, 35])
+def test_block_of_vectors(native, nv):
+    """Several vectors per application (35: more than one vector per slab of the final sum) against one at a time."""
+    from itofoggysim_b200 import solver
+    sc = scene([12, 5, 17, 9, 12, 12, 8], 3, 8)
+    g = scale(sc)
+    rng = np.random.default_rng(nv)
+    X = (rng.standard_normal((nv, g.size)) + 1j * rng.standard_normal((nv, g.size))) * g
+    with solver.MultiSphereSolver(sc, pair_tables=1) as s:
+        Y = s.calculate_vector_b_block(X) / g
+        for v in range(nv):
+            y = s.calculate_vector_b(X[v]) / g
+            assert np.abs(Y[v] - y).max() <= 1e-13 * np.abs(y).max()
+
+
+def test_mixed_handle_keeps_both_precisions(native):
+    """On a mixed-precision handle FP32 asked for by name and the FP64 steps do not disturb each other's tables."""
+    from itofoggysim_b200 import solver
+    sc = scene([12, 5, 17, 9, 12], 3, 9)
+    g = scale(sc)
+    x = np.random.default_rng(1).standard_normal(g.size) * g
+    with solver.MultiSphereSolver(sc, pair_tables=1, precision=1) as s:
+        y0 = s.calculate_vector_b(x)
+        f = s.calculate_vector_b_block(x[None], precision=1)[0]
+        y1 = s.calculate_vector_b(x)
+        assert np.array_equal(f, s.calculate_vector_b_block(x[None], precision=1)[0])
+    with solver.MultiSphereSolver(sc, pair_tables=1, precision=1) as s:
+        assert np.array_equal(f, s.calculate_vector_b_block(x[None], precision=1)[0])   # FP32 tables first
+        y2 = s.calculate_vector_b(x)
+    assert np.array_equal(y0, y1) and np.array_equal(y0, y2)
+    assert 0.0 < np.abs((f - y0) / g).max() <= 1e-5 * np.abs(y0 / g).max()
