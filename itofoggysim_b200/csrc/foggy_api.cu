@@ -2135,11 +2135,12 @@ int32_t foggy_get_field(foggy_handle h, const double* x, int32_t mem, int32_t np
     // per-call buffers: sphere radii, and the points and fields when they live on the host
     void* tmp = nullptr;
     const size_t np = (size_t)npoints;
-    size_t bytes = rad.size() * sizeof(double);
+    size_t bytes = (rad.size() + 1) / 2 * 2 * sizeof(double) + len * sizeof(cplx);
     if (mem == FOGGY_MEM_HOST) bytes += len * sizeof(cplx) + 3 * np * sizeof(double) + 6 * np * sizeof(cplx);
     CK(h, talloc(h, &tmp, bytes));
     double* d_rad = static_cast<double*>(tmp);
-    char* q = reinterpret_cast<char*>(d_rad + rad.size());
+    cplx* d_ab = reinterpret_cast<cplx*>(d_rad + (rad.size() + 1) / 2 * 2);
+    char* q = reinterpret_cast<char*>(d_ab + len);
     cudaError_t e = cudaMemcpyAsync(d_rad, rad.data(), rad.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream);
     if (mem == FOGGY_MEM_HOST) {
         cplx* xs = reinterpret_cast<cplx*>(q);
@@ -2153,8 +2154,16 @@ int32_t foggy_get_field(foggy_handle h, const double* x, int32_t mem, int32_t np
         pd = ps;
     }
     if (e == cudaSuccess) {
-        k_field<<<npoints, 128, 0, h->stream>>>(scene_view(h), d_rad, h->pg, C, xd, pd, e_field_0,
-                                                h->prm.n_medium / 299792458.0, ed, hd);
+        // warps per CTA: enough for 16 on every SM, no more than there are spheres or shared memory for
+        const int blocks = (npoints + 31) / 32;
+        int warps = std::max(1, std::min({16, h->N, (148 * 16 + blocks - 1) / blocks}));
+        warps = std::max(warps, std::min(4, h->N));
+        while (warps > 1 && field_smem_bytes(h->pg, 32 * warps) > ((size_t)200 << 10)) --warps;
+        const size_t smem = field_smem_bytes(h->pg, 32 * warps);
+        raise_smem_ceiling(reinterpret_cast<const void*>(k_field), smem);
+        k_field_coeff<<<h->N, 128, 0, h->stream>>>(C, xd, d_ab);
+        k_field<<<blocks, 32 * warps, smem, h->stream>>>(scene_view(h), d_rad, h->pg, C, d_ab, npoints, pd, e_field_0,
+                                                         h->prm.n_medium / 299792458.0, ed, hd);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && mem == FOGGY_MEM_HOST) {

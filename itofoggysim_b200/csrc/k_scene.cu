@@ -411,163 +411,221 @@ __global__ void k_cross_sections(SceneView sc, const cplx* x, const cplx* pq, do
 // libmath/src/math/lib_math_vector_spherical_harmonics.f90:132-419) -------------------------------
 //   E += sum_nm E_nm i (a_nm N_nm + b_nm M_nm),  H += n_medium / c0 sum_nm E_nm (b_nm N_nm + a_nm M_nm)
 //   E_nm = |E0| (2n+1) (n-m)!/(n+m)! i^n, with h_n^(1) in M, N, per sphere in its own frame,
-// converted to cartesian components and summed; zero at a point inside any sphere.  One CTA per
-// point, each thread a strided subset of the spheres; Legendre functions (no Condon-Shortley
-// phase), pi_nm = m P_n^m / sin t and tau_nm = dP_n^m/dt by recurrence per order m.
+// converted to cartesian components and summed; zero at a point inside any sphere.
+//
+// One thread per point, one warp per 32 points and subset of the spheres, the subsets of a CTA's warps added in
+// order: a warp's lanes share the sphere, so its coefficients are one broadcast load, and the radial functions
+// and Legendre rows sit in shared memory, one column per thread.  For each degree the angular sums over m,
+//   A_P, A_tau, A_pi = sum_m (P, tau, pi) a'_m e^{i m phi} and B likewise, +m and -m together,
+// come first and meet the radial factors once: 18 multiply-adds per coefficient, where forming M and N per (n, m)
+// took about 110.  FP64-pipe bound.  46600 points x 71 spheres of order 5: 3.6 -> 0.79 ms (one CTA per point with its
+// threads over the spheres before, 71 of 128 at work and the Bessel sequences in local memory).
 namespace {
-constexpr int kFieldThreads = 128;
-
-// contribution of degree n and order mm to the spherical components of E and H, given P_n^mm,
-// pi_n,mm, tau_n,mm and (n-mm)!/(n+mm)!
-__device__ __forceinline__ void field_term(int n, int mm, double P, double pv, double tv, double ratio, cplx zn,
-                                           cplx xid, double rho, cplx e, const cplx* a, const cplx* b, int base,
-                                           double e0, cplx* es, cplx* hs) {
-    const cplx Mt = mk(0.0, pv) * zn * e, Mp = (-tv) * (zn * e);
-    const cplx Nr = ((double)(n * (n + 1)) * P / rho) * (zn * e), Nt = (tv / rho) * (xid * e),
-               Np = (1.0 / rho) * (mk(0.0, pv) * (xid * e));
-    const cplx Enm = ipow_mul(n, mk(e0 * (2.0 * n + 1.0) * ratio, 0.0));
-    const cplx an = a[base + mm], bn = b[base + mm];
-    const cplx ie = mk(-Enm.y, Enm.x);   // i E_nm
-    es[0] = es[0] + ie * (an * Nr);
-    es[1] = es[1] + ie * (an * Nt + bn * Mt);
-    es[2] = es[2] + ie * (an * Np + bn * Mp);
-    hs[0] = hs[0] + Enm * (bn * Nr);
-    hs[1] = hs[1] + Enm * (bn * Nt + an * Mt);
-    hs[2] = hs[2] + Enm * (bn * Np + an * Mp);
+// j_n(x), n = 0..P, into out[n ld] (dev_sph_jn's recurrences with a stride)
+__device__ __forceinline__ void sph_jn_column(double x, int P, double* out, int ld) {
+    double s, c;
+    sincos(x, &s, &c);
+    const double rx = 1.0 / x;
+    const double j0 = s * rx, j1 = (s * rx - c) * rx;
+    if (x > (double)P) {
+        double a = j0, b = j1;
+        out[0] = j0;
+        for (int n = 1; n <= P; ++n) {
+            out[n * ld] = b;
+            const double t = (2.0 * n + 1.0) * rx * b - a;
+            a = b;
+            b = t;
+        }
+        return;
+    }
+    const int start = P + 16 + (int)x + (int)sqrt(40.0 * (P + x));
+    double fnp1 = 0.0, fn = 1e-300;
+    for (int n = start; n >= 1; --n) {
+        const double fnm1 = (2.0 * n + 1.0) * rx * fn - fnp1;
+        if (n - 1 <= P) out[(n - 1) * ld] = fnm1;
+        fnp1 = fn;
+        fn = fnm1;
+        if (fabs(fn) > 1e250) {
+            fn *= 1e-250;
+            fnp1 *= 1e-250;
+            for (int k = n - 1; k <= P; ++k) out[k * ld] *= 1e-250;
+        }
+    }
+    const double scale = (fabs(j0) >= fabs(j1)) ? j0 / out[0] : j1 / out[ld];
+    for (int n = 0; n <= P; ++n) out[n * ld] *= scale;
+}
+// s += r z
+__device__ __forceinline__ void axpy(cplx& s, double r, cplx z) {
+    s.x = fma(r, z.x, s.x);
+    s.y = fma(r, z.y, s.y);
 }
 }  // namespace
 
-__global__ void __launch_bounds__(kFieldThreads) k_field(SceneView sc, const double* radius_s, int pg, int C,
-                                                         const cplx* x, const double* pts, double e0,
-                                                         double h_factor, cplx* E_out, cplx* H_out) {
-    const int ip = blockIdx.x;
-    const int tid = threadIdx.x;
-    __shared__ int inside;
-    __shared__ double red[12][kFieldThreads];
-    if (tid == 0) inside = 0;
-    __syncthreads();
-    const double* pt = pts + 3 * (size_t)ip;
-    cplx acc[6];
-    for (int c = 0; c < 6; ++c) acc[c] = mk(0.0, 0.0);
-    double jb[2 * kMaxDegree + 4], yb[2 * kMaxDegree + 4];
-    for (int j = tid; j < sc.n; j += kFieldThreads) {
-        const double d0 = pt[0] - sc.centres[3 * (size_t)j];
-        const double d1 = pt[1] - sc.centres[3 * (size_t)j + 1];
-        const double d2 = pt[2] - sc.centres[3 * (size_t)j + 2];
+// The coefficients with what depends on (n, m) alone, a and b of one order side by side:
+// (n-m)!/(n+m)! for m >= 0, (-1)^m for m < 0 (there it cancels against P_n^{-m}).
+__global__ void k_field_coeff(int C, const cplx* x, cplx* ab) {
+    const size_t j = blockIdx.x;
+    for (int t = threadIdx.x; t < C; t += blockDim.x) {
+        int n, m;
+        decode_nm(t, n, m);
+        double f = (m & 1) ? -1.0 : 1.0;
+        if (m >= 0) {
+            f = 1.0;
+            for (int q = n - m + 1; q <= n + m; ++q) f *= (double)q;
+            f = 1.0 / f;
+        }
+        ab[2 * (j * C + t)] = f * x[2 * j * C + t];
+        ab[2 * (j * C + t) + 1] = f * x[2 * j * C + C + t];
+    }
+}
+
+__global__ void __launch_bounds__(512) k_field(SceneView sc, const double* radius_s, int pg, int C, const cplx* ab,
+                                               int npoints, const double* pts, double e0, double h_factor, cplx* E_out,
+                                               cplx* H_out) {
+    extern __shared__ __align__(16) double field_smem[];
+    const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = T >> 5;
+    double* jb = field_smem + tid;                  // [pg + 2] j_n
+    double* q1 = jb + (size_t)(pg + 2) * T;         // [pg + 1] Q_{n-1}^m (order 0: P_{n-1})
+    double* q2 = q1 + (size_t)(pg + 1) * T;         // [pg + 1] of n - 2
+    const int ip = blockIdx.x * 32 + lane;
+    const int pi_ = ip < npoints ? ip : npoints - 1;
+    const double p0 = pts[3 * (size_t)pi_], p1 = pts[3 * (size_t)pi_ + 1], p2 = pts[3 * (size_t)pi_ + 2];
+    bool inside = false;
+    double acc[12];
+#pragma unroll
+    for (int c = 0; c < 12; ++c) acc[c] = 0.0;
+    for (int j = warp; j < sc.n; j += warps) {
+        const double d0 = p0 - sc.centres[3 * (size_t)j];
+        const double d1 = p1 - sc.centres[3 * (size_t)j + 1];
+        const double d2 = p2 - sc.centres[3 * (size_t)j + 2];
         const double r = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
         if (!(r > radius_s[j])) {
-            inside = 1;
+            inside = true;
             continue;
         }
         if (!(e0 > 1e-200)) continue;
-        const double th = (r == 0.0) ? 0.0 : acos(d2 / r);
-        const double ph = (d0 == 0.0 && d1 == 0.0) ? 0.0 : atan2(d1, d0);
-        const double rho = sc.k * r;
-        dev_sph_jn(rho, pg + 1, jb);
-        dev_sph_yn(rho, pg + 1, yb);
-        const double xc = cos(th), st = sin(th);
-        const bool pole = (xc == 1.0 || xc == -1.0);
-        const cplx* a = x + (size_t)2 * C * j;
-        const cplx* b = a + C;
-        cplx es[3] = {mk(0, 0), mk(0, 0), mk(0, 0)}, hs[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
-        // Q_n^m = P_n^m / sin t by the LPMNS recurrence; pi_nm = m Q_n^m, tau_nm = n x Q_n^m - (n+m) Q_{n-1}^m,
-        // tau_n0 = -P_n^1 = -sin t Q_n^1; negative orders from P_n^{-m} = f P_n^m, f = (-1)^m (n-m)!/(n+m)!
-        // (pi_{n,-m} = -f pi_nm, tau_{n,-m} = f tau_nm); at the poles the reference's table
-        // (lib_math_legendre.f90:854-920, without the phase)
-        double fact2m = 1.0;   // (2m)!
-        for (int m = 0; m <= pg; ++m) {
-            if (m > 0) fact2m *= (2.0 * m - 1.0) * (2.0 * m);
-            double sphi, cphi;
-            sincos((double)m * ph, &sphi, &cphi);
-            const cplx ep = mk(cphi, sphi), em = mk(cphi, -sphi);
-            const int mq = m == 0 ? 1 : m;   // order of the Q sequence (Q^1 for tau_n0)
-            double qmm = 1.0;
-            for (int q = 1; q <= mq; ++q) qmm *= (2.0 * q - 1.0);
-            for (int q = 1; q < mq; ++q) qmm *= st;
-            double qc = qmm, qprev = 0.0;                       // Q_n^mq at n = mq, and n - 1
-            double pc = m == 0 ? 1.0 : qmm * st, pprev = 0.0;   // P_n^m at n = m, and n - 1
-            double fr = 1.0 / fact2m;                           // (n-m)!/(n+m)! at n = m
-            int nq = mq, np_ = m;
-            for (int n = max(m, 1); n <= pg; ++n) {
-                while (np_ < n) {   // advance P_n^m and (n-m)!/(n+m)!
-                    ++np_;
-                    const double pn = ((2.0 * np_ - 1.0) * xc * pc - (np_ + m - 1.0) * pprev) / (np_ - m);
-                    pprev = pc;
-                    pc = pn;
-                    fr *= (double)(np_ - m) / (double)(np_ + m);
-                }
-                while (nq < n) {    // advance Q_n^mq
-                    ++nq;
-                    const double qn = ((2.0 * nq - 1.0) * xc * qc - (nq + mq - 1.0) * qprev) / (nq - mq);
-                    qprev = qc;
-                    qc = qn;
-                }
-                const cplx zn = mk(jb[n], yb[n]);
-                const cplx zm1 = mk(jb[n - 1], yb[n - 1]), zp1 = mk(jb[n + 1], yb[n + 1]);
-                const cplx xid = 0.5 * (rho * zm1 + zn - rho * zp1);
-                const int base = n * n - 1 + n;
-                if (m == 0) {
-                    const double P0 = pole ? ((xc < 0.0 && (n & 1)) ? -1.0 : 1.0) : pc;
-                    const double t0 = pole ? 0.0 : -st * qc;
-                    field_term(n, 0, P0, 0.0, t0, 1.0, zn, xid, rho, ep, a, b, base, e0, es, hs);
-                    continue;
-                }
-                double pip, taup, pim, taum, Pp, Pm;
-                if (pole) {
-                    Pp = Pm = 0.0;
-                    pip = taup = pim = taum = 0.0;
-                    if (m == 1) {
-                        const double N2 = (double)(n * (n + 1) / 2);
-                        if (xc > 0.0) {
-                            pip = N2; pim = 0.5; taup = N2; taum = -0.5;
-                        } else if ((n & 1) == 0) {
-                            pip = -N2; pim = -0.5; taup = N2; taum = -0.5;
-                        } else {
-                            pip = N2; pim = 0.5; taup = -N2; taum = -0.5;
-                        }
-                    }
-                } else {
-                    const double f = (m & 1) ? -fr : fr;
-                    Pp = pc;
-                    Pm = f * pc;
-                    pip = m * qc;
-                    taup = n * xc * qc - (n + m) * qprev;
-                    pim = -f * pip;
-                    taum = f * taup;
-                }
-                field_term(n, m, Pp, pip, taup, fr, zn, xid, rho, ep, a, b, base, e0, es, hs);
-                field_term(n, -m, Pm, pim, taum, 1.0 / fr, zn, xid, rho, em, a, b, base, e0, es, hs);
-            }
+        const double th = acos(d2 / r);
+        double st, xc;
+        sincos(th, &st, &xc);
+        // the reference's pole table (lib_math_legendre.f90:854-920, without the phase): the limits of the general
+        // functions, but for tau_{n,-1} of odd n at theta = pi, which has the opposite sign
+        const bool pole = xc == 1.0 || xc == -1.0;
+        const bool south = xc == -1.0;
+        if (pole) st = 0.0;
+        double sp = 0.0, cp = 1.0;
+        if (d0 != 0.0 || d1 != 0.0) {
+            const double m = fmax(fabs(d0), fabs(d1)), a = d0 / m, b = d1 / m, h = sqrt(a * a + b * b);
+            cp = a / h;
+            sp = b / h;
         }
-        const double ct = xc, cp = cos(ph), sp = sin(ph);
-        const cplx ex = st * cp * es[0] + ct * cp * es[1] - sp * es[2];
-        const cplx ey = st * sp * es[0] + ct * sp * es[1] + cp * es[2];
-        const cplx ez = ct * es[0] - st * es[1];
-        const cplx hx = st * cp * hs[0] + ct * cp * hs[1] - sp * hs[2];
-        const cplx hy = st * sp * hs[0] + ct * sp * hs[1] + cp * hs[2];
-        const cplx hz = ct * hs[0] - st * hs[1];
-        acc[0] = acc[0] + ex;
-        acc[1] = acc[1] + ey;
-        acc[2] = acc[2] + ez;
-        acc[3] = acc[3] + h_factor * hx;
-        acc[4] = acc[4] + h_factor * hy;
-        acc[5] = acc[5] + h_factor * hz;
+        const double rho = sc.k * r, rr = 1.0 / rho;
+        sph_jn_column(rho, pg + 1, jb, T);
+        // y_{n-1}, y_n upwards (dev_sph_yn)
+        double sr, cr;
+        sincos(rho, &sr, &cr);
+        double ym = -cr * rr, y = (-cr * rr - sr) * rr;
+        double qmm = 1.0;                               // Q_n^n = (2n-1)!! sin^{n-1}
+        q1[0] = 1.0;                                    // P_0
+        q2[0] = 0.0;
+        cplx es[3] = {mk(0, 0), mk(0, 0), mk(0, 0)}, hs[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
+        const cplx* cj = ab + 2 * (size_t)j * C;
+        for (int n = 1; n <= pg; ++n) {
+            cplx aP = mk(0, 0), aT = mk(0, 0), aQ = mk(0, 0), bP = mk(0, 0), bT = mk(0, 0), bQ = mk(0, 0);
+            const cplx* cn = cj + 2 * (n * n - 1 + n);
+            if (n > 1) qmm *= (2.0 * n - 1.0) * st;
+            cplx e = mk(cp, sp);
+            for (int m = 1; m <= n; ++m) {
+                // Q_n^m = P_n^m / sin t by the LPMNS recurrence; pi = m Q, tau = n x Q_n - (n + m) Q_{n-1}
+                double q, qp = 0.0;
+                if (m == n) {
+                    q = qmm;
+                } else {
+                    qp = q1[m * T];
+                    const double qpp = m == n - 1 ? 0.0 : q2[m * T];
+                    q = ((2.0 * n - 1.0) * xc * qp - (n + m - 1.0) * qpp) / (double)(n - m);
+                    q2[m * T] = qp;
+                }
+                q1[m * T] = q;
+                const double P = q * st, pv = m * q, tv = n * xc * q - (n + m) * qp;
+                const cplx ap = cn[2 * m], bp = cn[2 * m + 1], am = cn[-2 * m], bm = cn[-2 * m + 1];
+                const cplx ga = e * ap, gb = e * bp, ha = conjg(e) * am, hb = conjg(e) * bm;
+                const cplx sa = ga + ha, da = ga - ha, sb = gb + hb, db = gb - hb;
+                const bool odd_south = south && m == 1 && (n & 1);
+                axpy(aP, P, sa);
+                axpy(aT, tv, odd_south ? da : sa);
+                axpy(aQ, pv, da);
+                axpy(bP, P, sb);
+                axpy(bT, tv, odd_south ? db : sb);
+                axpy(bQ, pv, db);
+                if (m < n) e = e * mk(cp, sp);
+                if (m == 1) {
+                    // order 0: tau = -P_n^1
+                    const cplx a0 = cn[0], b0 = cn[1];
+                    const double pm = q1[0], pn = ((2.0 * n - 1.0) * xc * pm - (n - 1.0) * q2[0]) / (double)n;
+                    q2[0] = pm;
+                    q1[0] = pn;
+                    const double P0 = pole ? ((south && (n & 1)) ? -1.0 : 1.0) : pn, t0 = -P;
+                    axpy(aP, P0, a0);
+                    axpy(aT, t0, a0);
+                    axpy(bP, P0, b0);
+                    axpy(bT, t0, b0);
+                }
+            }
+            const double yp = (2.0 * n + 1.0) * rr * y - ym;   // y_{n+1}
+            const cplx zn = mk(jb[n * T], y), zm = mk(jb[(n - 1) * T], ym), zp = mk(jb[(n + 1) * T], yp);
+            ym = y;
+            y = yp;
+            const double f = e0 * (2.0 * n + 1.0);
+            const cplx W = ipow_mul(n, f * zn);
+            const cplx V = ipow_mul(n, (f * rr) * (0.5 * (rho * zm + zn - rho * zp)));
+            const cplx Wr = ((double)(n * (n + 1)) * rr) * W;
+            auto im = [](cplx z) { return mk(-z.y, z.x); };
+            es[0] = es[0] + Wr * aP;
+            es[1] = es[1] + (V * aT + W * im(bQ));
+            es[2] = es[2] + (V * im(aQ) - W * bT);
+            hs[0] = hs[0] + Wr * bP;
+            hs[1] = hs[1] + (V * bT + W * im(aQ));
+            hs[2] = hs[2] + (V * im(bQ) - W * aT);
+        }
+        // to cartesian components; E carries another i
+        auto add = [&](const cplx* v, double* o) {
+            const cplx x_ = st * cp * v[0] + xc * cp * v[1] - sp * v[2];
+            const cplx y_ = st * sp * v[0] + xc * sp * v[1] + cp * v[2];
+            const cplx z_ = xc * v[0] - st * v[1];
+            o[0] += x_.x;
+            o[1] += x_.y;
+            o[2] += y_.x;
+            o[3] += y_.y;
+            o[4] += z_.x;
+            o[5] += z_.y;
+        };
+        add(es, acc);
+        add(hs, acc + 6);
     }
-    for (int c = 0; c < 6; ++c) {
-        red[2 * c][tid] = acc[c].x;
-        red[2 * c + 1][tid] = acc[c].y;
-    }
+    // the warps' sums in order, through shared memory (one component at a time: one value per thread)
+    double* red = field_smem;
     __syncthreads();
-    for (int s_ = kFieldThreads / 2; s_ > 0; s_ >>= 1) {
-        if (tid < s_)
-            for (int c = 0; c < 12; ++c) red[c][tid] += red[c][tid + s_];
+    red[tid] = inside ? 1.0 : 0.0;
+    __syncthreads();
+    bool in = false;
+    for (int w = 0; w < warps; ++w) in |= red[w * 32 + lane] != 0.0;
+    double sum[12];
+    for (int c = 0; c < 12; ++c) {
         __syncthreads();
+        red[tid] = acc[c];
+        __syncthreads();
+        double v = 0.0;
+        for (int w = 0; w < warps; ++w) v += red[w * 32 + lane];
+        sum[c] = in ? 0.0 : v;
     }
-    if (tid < 6) {
-        const cplx v = inside ? mk(0.0, 0.0) : mk(red[2 * tid][0], red[2 * tid + 1][0]);
-        if (tid < 3) E_out[3 * (size_t)ip + tid] = v;
-        else H_out[3 * (size_t)ip + tid - 3] = v;
+    if (warp == 0 && ip < npoints) {
+        for (int c = 0; c < 3; ++c) {
+            E_out[3 * (size_t)ip + c] = mk(-sum[2 * c + 1], sum[2 * c]);
+            H_out[3 * (size_t)ip + c] = mk(h_factor * sum[6 + 2 * c], h_factor * sum[6 + 2 * c + 1]);
+        }
     }
 }
+
+size_t field_smem_bytes(int pg, int threads) { return (size_t)threads * (3 * pg + 4) * sizeof(double); }
 
 }  // namespace foggy
