@@ -180,6 +180,7 @@ struct foggy_handle_s {
     int64_t* d_fmm_taboff = nullptr; // per list entry, its block's offset in d_fmm_tab
     cplxf* d_fmm_tab32 = nullptr;    // the blocks in single precision (mixed-precision solves)
     bool fmm_tab_ready = false;
+    std::vector<int> fmm_order;      // box order of each level
     int fmm_pmax = 0;                // largest box order (the global order, or per-level orders)
     std::vector<int> fmm_list_host;  // the twelve pass lists, read back once (chunk counts)
     int fmm_tab_key[5] = {0, 0, 0, 0, 0};   // (convention, z_coupling, z_translation_gt_r, on, precision)
@@ -889,6 +890,8 @@ void free_fmm(foggy_handle h) {
 // few boxes still fill the GPU; their partial sums need fewer than 2 kFmmFill slabs of one target.
 constexpr int kFmmFill = 148 * 6;
 constexpr int kFmmChunks = 16;
+// list entries from which a pass runs on the tensor cores
+constexpr int kFmmMmaEntries = 4096;
 
 // Expansion order of the boxes of level l.  The reference expands every box to its global order
 // p_g (digits = 0).  With digits > 0: the excess-bandwidth order L = kd + 1.8 digits^(2/3) (kd)^(1/3)
@@ -1071,6 +1074,7 @@ int ensure_fmm(foggy_handle h) {
         pmax = std::max(pmax, L);
     }
     h->fmm_pmax = pmax;
+    h->fmm_order.assign(lv.order, lv.order + nlev);
     const int Pm = pmax * (pmax + 2);
     int rc = ensure_tables(h, pmax);
     if (!rc) rc = dalloc(h, &h->d_fmm_c, 3 * (size_t)nbox);
@@ -1298,7 +1302,6 @@ int apply_operator_fmm(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false
     add(4, S, B, h->d_fmm_D, h->d_fmm_slab, 8, 9, 0, h->N, sts, z_dor, 0, conv == 0);
     add(5, S, S, x, h->d_fmm_slab + h->n_unk, 10, 11, 0, h->N, 1.0, zi, 0, false);
     TRY(ensure_fmm_tables(h, base, passes));
-    const bool tabs = h->d_fmm_taboff != nullptr && (!fp32 || h->d_fmm_tab32 != nullptr);
     // the near field needs only x: it runs on a second stream beside the box passes
     if (!h->side) {
         if (cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1309,28 +1312,59 @@ int apply_operator_fmm(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false
     CK(h, cudaEventRecord(h->ev_fork, h->stream));
     CK(h, cudaStreamWaitEvent(h->side, h->ev_fork, 0));
     Trace tr(fp32 ? "ML-FMM operator (FP32)" : "ML-FMM operator");
-    for (size_t i = 0; i < passes.size(); ++i) {
-        const FmmPass& q = passes[i];
-        const bool near = stage[i] == 5;
-        Trace tp(names[stage[i]]);
+    // One launch of a pass; returns the entries of its lists.  Passes with few targets split each target's sources over
+    // several CTAs, no more than the longest of its source lists (in batches of four on the tensor cores).
+    auto list_of = [&](const FmmPass& q, int& longest) {
+        const int* ptr = h->fmm_list_host.data() + h->fmm_lofs[q.lp] + (q.lp == 0 || q.lp >= 8 ? 0 : q.tbase);
+        longest = 0;
+        for (int b = 0; b < q.ntgt; ++b) longest = std::max(longest, ptr[b + 1] - ptr[b]);
+        return q.ntgt > 0 ? ptr[q.ntgt] - ptr[0] : 0;
+    };
+    auto launch = [&](const FmmPass& q, bool near, int pp_mma) {
+        if (q.ntgt <= 0) return;
         TransArgs a = fmm_pass_args(h, base, q);
         if (near) a.slab = h->d_fmm_chunks2;
-        if (tabs) {
+        if (h->d_fmm_taboff) {
             a.tab = h->d_fmm_tab;
             a.tab32 = h->d_fmm_tab32;
             a.tab_off = h->d_fmm_taboff + h->fmm_lofs[q.li];
         }
-        // passes with few targets split each target's sources over several CTAs, no more than the
-        // longest of its source lists
+        if (fp32 && !h->d_fmm_tab32 && !pp_mma) a.tab_off = nullptr;
         int longest = 0;
-        if (q.ntgt > 0) {
-            const int* ptr = h->fmm_list_host.data() + h->fmm_lofs[q.lp] + (q.lp == 0 || q.lp >= 8 ? 0 : q.tbase);
-            for (int b = 0; b < q.ntgt; ++b) longest = std::max(longest, ptr[b + 1] - ptr[b]);
+        list_of(q, longest);
+        if (pp_mma) longest = (longest + 3) / 4;
+        const int chunks = std::max(1, std::min({kFmmChunks, (kFmmFill + q.ntgt - 1) / q.ntgt, longest}));
+        cudaStream_t st = near ? h->side : h->stream;
+        if (pp_mma) launch_translate_mma(a, mma_tabs(h), pp_mma, q.ntgt, chunks, st);
+        else launch_translate(a, q.ntgt, chunks, st);
+        h->launches += chunks > 1 ? 2 : 1;
+    };
+    // On the tensor cores: cached blocks, orders up to kMmaDegree, lists of four sources and more (a shorter list
+    // leaves units of its batch empty) and enough of them that the pass is not its launch's latency alone.
+    auto takes_mma = [&](const FmmPass& q, int pp) {
+        int longest = 0;
+        const int entries = list_of(q, longest);
+        return h->d_fmm_taboff && pp <= kMmaDegree && entries >= 4 * q.ntgt && entries >= kFmmMmaEntries;
+    };
+    for (size_t i = 0; i < passes.size(); ++i) {
+        const FmmPass& q = passes[i];
+        Trace tp(names[stage[i]]);
+        if (stage[i] == 2) {
+            // M2L: one launch, unless its size pays for one per level with that level's order
+            int longest = 0;
+            if (h->d_fmm_taboff && list_of(q, longest) >= kFmmMmaEntries) {
+                for (int li = 0; li < nlev; ++li) {
+                    FmmPass ql = q;
+                    ql.tbase = t.level_base[li];
+                    ql.ntgt = t.level_base[li + 1] - ql.tbase;
+                    const int pp = h->fmm_order[li];
+                    launch(ql, false, takes_mma(ql, pp) ? pp : 0);
+                }
+                continue;
+            }
         }
-        const int chunks =
-            q.ntgt > 0 ? std::max(1, std::min({kFmmChunks, (kFmmFill + q.ntgt - 1) / q.ntgt, longest})) : 1;
-        launch_translate(a, q.ntgt, chunks, near ? h->side : h->stream);
-        if (q.ntgt > 0) h->launches += chunks > 1 ? 2 : 1;
+        const int pp = stage[i] == 5 ? std::max(h->pmax, 1) : base.pp;
+        launch(q, stage[i] == 5, (stage[i] == 5 && takes_mma(q, pp)) ? pp : 0);
     }
     // join first, so that whatever follows on the handle's stream (frees included) comes after the side
     cudaEventRecord(h->ev_join, h->side);

@@ -246,6 +246,9 @@ __global__ void k_fmm_tab(const FmmTabEntry* u, SGaunt g, int z, cplx* tab);
 // one pass: ntargets x chunks CTAs (chunks >= 1; with several, slab must hold chunks x ntargets x
 // slab_ld entries)
 void launch_translate(const TransArgs& a, int ntargets, int chunks, cudaStream_t s);
+void launch_translate_sum(const TransArgs& a, int ntargets, int chunks, cudaStream_t s);
+// the same on the FP64 tensor cores: a.tab given, orders of targets and sources <= pp <= kMmaDegree
+void launch_translate_mma(const TransArgs& a, const MmaTabs& mt, int pp, int ntargets, int chunks, cudaStream_t s);
 // single-pair translation for the parity entry point: A, B blocks in the scaled basis
 __global__ void k_translation_pair(AxialView ax, DTabs dt, double x, double theta, double phi, int pn, int pnu,
                                    int z, cplx* A, cplx* B);

@@ -881,7 +881,8 @@ __global__ void k_fmm_rho(TransArgs a, double* rho, int2* deg) {
 // One coaxial block per distinct (rho, target degree, source degree) of a pass: S(k; mu, n) summed
 // from the scalar Gaunt table exactly as the translation stage sums it without tables (radial
 // functions to degree p_t + p_s + 1, the same terms in the same order), on the square layout of
-// the pair tables; entries the translation never reads (mu > p_s + 1 or n > p_t) are zero.
+// the pair tables, both halves of the square (the tensor-core passes read along mu); entries neither reading takes
+// (degrees above p_s + 1 and p_t, or above p_t and p_s + 1) are zero.
 __global__ void __launch_bounds__(256) k_fmm_tab(const FmmTabEntry* u, SGaunt g, int z, cplx* tab) {
     __shared__ double jb[2 * kMaxDegree + 8], yb[2 * kMaxDegree + 8];
     __shared__ cplx zeta[2 * kMaxDegree + 8];
@@ -906,7 +907,7 @@ __global__ void __launch_bounds__(256) k_fmm_tab(const FmmTabEntry* u, SGaunt g,
         const int64_t r = q - pair_block_offset(k, M2, M2);
         const int cols = M2 - k;
         const int mu = k + (int)(r / cols), n = k + (int)(r % cols);
-        if (mu > e.ps + 1 || n > e.pt) {
+        if ((mu > e.ps + 1 || n > e.pt) && (n > e.ps + 1 || mu > e.pt)) {
             out[q] = mk(0, 0);
             continue;
         }
@@ -964,7 +965,11 @@ void launch_translate(const TransArgs& a, int ntargets, int chunks, cudaStream_t
         raise_smem_ceiling(reinterpret_cast<const void*>(k_translate<cplx>), smem);
         k_translate<cplx><<<dim3(ntargets, chunks), kThreads, smem, s>>>(a);
     }
-    if (chunks > 1) k_translate_sum<<<ntargets, 256, 0, s>>>(a, chunks);
+    if (chunks > 1) launch_translate_sum(a, ntargets, chunks, s);
+}
+
+void launch_translate_sum(const TransArgs& a, int ntargets, int chunks, cudaStream_t s) {
+    k_translate_sum<<<ntargets, 256, 0, s>>>(a, chunks);
 }
 
 // ---------------------------------------------------------------------------------------------

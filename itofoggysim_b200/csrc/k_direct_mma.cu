@@ -1,5 +1,5 @@
-// The FP64 direct operator on the tensor cores (k_mma.cuh): one CTA per target sphere and chunk of a
-// source bucket, four sources per batch.  Same launches, slabs and result layout as k_direct.
+// FP64 translations on the tensor cores (k_mma.cuh): one CTA per target and chunk of its sources, four sources per
+// batch.  The direct operator (k_direct's launches and slabs) and the ML-FMM's passes over long lists.
 #include <cmath>
 
 #include "k_mma.cuh"
@@ -9,47 +9,33 @@ namespace foggy {
 namespace {
 using namespace mma;
 
-// direction of the translation from source l to target j, t = k (d_l - d_j), rounded as in disp_vec
-__device__ inline Dir pair_dir(const SceneView& sc, int j, int l) {
-    const double* ct = sc.centres + 3 * (size_t)j;
-    const double* cs = sc.centres + 3 * (size_t)l;
-    const double d0 = __dmul_rn(sc.k, __dsub_rn(cs[0], ct[0]));
-    const double d1 = __dmul_rn(sc.k, __dsub_rn(cs[1], ct[1]));
-    const double d2 = __dmul_rn(sc.k, __dsub_rn(cs[2], ct[2]));
+// direction of a translation, rounded as in disp_vec (k_direct.cu): t = k (sign (c_s - c_t) + sh)
+__device__ inline Dir pair_dir(const double* ct, const double* cs, double k, double sign, double sh0, double sh1,
+                               double sh2) {
+    const double d0 = __dmul_rn(k, __fma_rn(sign, __dsub_rn(cs[0], ct[0]), sh0));
+    const double d1 = __dmul_rn(k, __fma_rn(sign, __dsub_rn(cs[1], ct[1]), sh1));
+    const double d2 = __dmul_rn(k, __fma_rn(sign, __dsub_rn(cs[2], ct[2]), sh2));
     return direction(d0, d1, d2, sqrt(__fma_rn(d0, d0, __fma_rn(d1, d1, __dmul_rn(d2, d2)))));
 }
-
 // records are made once in eight batches: a call keeps their arithmetic out of the loop's code
-__device__ __noinline__ Dir pair_dir_call(const SceneView& sc, int j, int l) { return pair_dir(sc, j, l); }
-}  // namespace
+__device__ __noinline__ Dir pair_dir_call(const double* ct, const double* cs, double k, double sign, double sh0,
+                                          double sh1, double sh2) {
+    return pair_dir(ct, cs, k, sign, sh0, sh1, sh2);
+}
 
-template <int NI, int W, int CTAS>
-__global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTabs mt, DirectBucket bk, int us, int nrhs,
-                                                             int64_t ld, int per_rhs) {
-    extern __shared__ __align__(16) double smem_d[];
-    const SceneView& sc = a.sc;
-    // right-hand side fastest: the CTAs that read one pair's coaxial block run together
-    const int rhs = blockIdx.x % nrhs, j = bk.targets[blockIdx.x / nrhs];
-    if (!sc.couple[j]) return;
-    const cplx* const x = a.x + rhs * ld;
+// The translations of one target of degree pj, `mine` batches of four units; unit(i, l, un, dir) fills the record of unit
+// i of this CTA's batches, or leaves it empty.  The sums are in s.acc at the end, visible to every thread.
+template <int NI, int W, class UnitOf>
+__device__ __forceinline__ void run_batches(const Shared& s, const MmaTabs& mt, int pp, int pj, int mine, UnitOf unit) {
     constexpr int T = 32 * W, LD = phase_ld<NI>();
-    const int pp = bk.pp, c = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const Shared s = carve<NI>(smem_d, pp, us);
-    const int pj = sc.p[j], Pj = pj * (pj + 2);
-    const int nb = (bk.nsources + kUnits - 1) / kUnits;   // batches of the bucket; this CTA: c, c + chunks, ...
-
+    const int Pj = pj * (pj + 2);
     // records of this CTA's batches 8g..8g+7, one unit per lane (one warp)
     auto records = [&](int g) {
-        const int b = c + (8 * g + lane / kUnits) * bk.chunks, i = kUnits * b + lane % kUnits;
-        const int l = (b < nb && i < bk.nsources) ? bk.sources[i] : j;
         Dir d{1.0, 0.0, 1.0, 0.0, 1.0};
         Unit un{nullptr, nullptr, 0, -1, 1.0};
-        if (l != j) {
-            un.x = reinterpret_cast<const double2*>(x + sc.off[l]);
-            un.s = reinterpret_cast<const double2*>(a.pt.stab + a.pt.pair_off[pair_index(min(j, l), max(j, l), sc.n)]);
-            un.p = sc.p[l];
-            d = pair_dir_call(sc, j, l);
+        unit(kRecs * g + lane, un, d);
+        if (un.x) {
             un.rho = d.rho;
             un.km = d.rho == 0.0 ? -1 : min(pj, un.p);
         }
@@ -76,8 +62,8 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTa
                 const Unit& un = s.un[at + u];
                 const int M2 = max(pj, un.p) + 2;
                 if (lane <= un.km) {
-                    // rows mu = k..pl + 1 of the order's square block: 16-byte entries, so aligned
-                    const unsigned bytes = (unsigned)((un.p + 2 - lane) * (M2 - lane) * sizeof(cplx));
+                    // the order's square block up to the last row of either reading: 16-byte entries, so aligned
+                    const unsigned bytes = (unsigned)((pj + 1 - lane) * (M2 - lane) * sizeof(cplx));
                     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(un.s + block_offset(lane, M2)),
                                  "r"(bytes)
                                  : "memory");
@@ -96,7 +82,6 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTa
     const Lane<NI> L(s, pp, lane);
     __syncthreads();
     int cur = 0;
-    const int mine = c < nb ? (nb - c + bk.chunks - 1) / bk.chunks : 0;   // batches of this CTA
     for (int ib = 0; ib < mine; ++ib, cur ^= 1) {
         const Unit* un = s.un + slot(ib);
         const int pl4 = max(max(un[0].p, un[1].p), max(un[2].p, un[3].p));
@@ -134,23 +119,94 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTa
         }
     }
     __syncthreads();
+}
+
+// batches c, c + chunks, ... of a list of n units
+__device__ __forceinline__ int batches_of(int n, int c, int chunks) {
+    const int nb = (n + kUnits - 1) / kUnits;
+    return c < nb ? (nb - c + chunks - 1) / chunks : 0;
+}
+}  // namespace
+
+template <int NI, int W, int CTAS>
+__global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTabs mt, DirectBucket bk, int us, int nrhs,
+                                                             int64_t ld, int per_rhs) {
+    extern __shared__ __align__(16) double smem_d[];
+    const SceneView& sc = a.sc;
+    // right-hand side fastest: the CTAs that read one pair's coaxial block run together
+    const int rhs = blockIdx.x % nrhs, j = bk.targets[blockIdx.x / nrhs];
+    if (!sc.couple[j]) return;
+    const cplx* const x = a.x + rhs * ld;
+    const int c = blockIdx.y, pj = sc.p[j];
+    const Shared s = carve<NI>(smem_d, bk.pp, us);
+    run_batches<NI, W>(s, mt, bk.pp, pj, batches_of(bk.nsources, c, bk.chunks), [&](int r, Unit& un, Dir& d) {
+        const int i = kUnits * (c + r / kUnits * bk.chunks) + r % kUnits;
+        const int l = i < bk.nsources ? bk.sources[i] : j;
+        if (l == j) return;
+        un.x = reinterpret_cast<const double2*>(x + sc.off[l]);
+        un.s = reinterpret_cast<const double2*>(a.pt.stab + a.pt.pair_off[pair_index(min(j, l), max(j, l), sc.n)]);
+        un.p = sc.p[l];
+        d = pair_dir_call(sc.centres + 3 * (size_t)j, sc.centres + 3 * (size_t)l, sc.k, 1.0, 0.0, 0.0, 0.0);
+    });
     cplx* out = a.partial + ((size_t)rhs * per_rhs + bk.slab + c) * a.n_unk + sc.off[j];
-    for (int t = tid; t < 2 * Pj; t += T) out[t] = mk(s.acc[t].x, s.acc[t].y);
+    for (int t = threadIdx.x; t < 2 * pj * (pj + 2); t += 32 * W) out[t] = mk(s.acc[t].x, s.acc[t].y);
+}
+
+// One ML-FMM pass over cached blocks (k_translate's arguments and results)
+template <int NI, int W, int CTAS>
+__global__ void __launch_bounds__(32 * W, CTAS) k_translate_mma(TransArgs a, MmaTabs mt, int pp, int us) {
+    extern __shared__ __align__(16) double smem_d[];
+    const int t = a.tbase + blockIdx.x, c = blockIdx.y, chunks = gridDim.y;
+    const int pj = a.tgt.p[t];
+    const int i0 = a.lptr[blockIdx.x], n = a.lptr[blockIdx.x + 1] - i0;
+    const Shared s = carve<NI>(smem_d, pp, us);
+    run_batches<NI, W>(s, mt, pp, pj, batches_of(n, c, chunks), [&](int r, Unit& un, Dir& d) {
+        const int i = kUnits * (c + r / kUnits * chunks) + r % kUnits;
+        if (i >= n) return;
+        const int l = a.lidx[i0 + i];
+        un.x = reinterpret_cast<const double2*>(a.x + a.src.off[l]);
+        un.s = reinterpret_cast<const double2*>(a.tab + a.tab_off[i0 + i]);
+        un.p = a.src.p[l];
+        d = pair_dir_call(a.tgt.c + 3 * (size_t)t, a.src.c + 3 * (size_t)l, a.k, a.sign, a.sh[0], a.sh[1], a.sh[2]);
+    });
+    cplx* out = chunks == 1 ? a.out + a.tgt.off[t] : a.slab + ((size_t)c * gridDim.x + blockIdx.x) * a.slab_ld;
+    const bool add = a.add && chunks == 1;
+    for (int e = threadIdx.x; e < 2 * pj * (pj + 2); e += 32 * W) {
+        const cplx v = mk(s.acc[e].x, s.acc[e].y);
+        out[e] = add ? out[e] + v : v;
+    }
 }
 
 int mma_ctas_per_sm(int pp) { return pp <= 7 ? 4 : pp <= 23 ? 2 : 1; }
 
+// f(kernel tag) with the instantiation of a launch of largest degree pp
+template <class F>
+static void by_degree(int pp, F f) {
+    if (pp <= 7) f.template operator()<1, mma::warps_of(7), 4>();
+    else if (pp <= 15) f.template operator()<2, mma::warps_of(15), 2>();
+    else if (pp <= 23) f.template operator()<3, mma::warps_of(23), 2>();
+    else f.template operator()<4, mma::warps_of(31), 1>();
+}
+
 void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, int nrhs, int64_t ld, int per_rhs,
                        cudaStream_t s) {
-    auto go = [&](auto kernel, size_t smem) {
+    by_degree(b.pp, [&]<int NI, int W, int CTAS>() {
+        auto* kernel = k_direct_mma<NI, W, CTAS>;
+        const size_t smem = mma::smem_bytes<NI>(b.pp);
         raise_smem_ceiling(reinterpret_cast<const void*>(kernel), smem);
-        kernel<<<dim3((unsigned)b.ntargets * nrhs, b.chunks), 32 * mma::warps_of(b.pp), smem, s>>>(
-            a, mt, b, mma::unit_size(b.pp), nrhs, ld, per_rhs);
-    };
-    if (b.pp <= 7) go(k_direct_mma<1, mma::warps_of(7), 4>, mma::smem_bytes<1>(b.pp));
-    else if (b.pp <= 15) go(k_direct_mma<2, mma::warps_of(15), 2>, mma::smem_bytes<2>(b.pp));
-    else if (b.pp <= 23) go(k_direct_mma<3, mma::warps_of(23), 2>, mma::smem_bytes<3>(b.pp));
-    else go(k_direct_mma<4, mma::warps_of(31), 1>, mma::smem_bytes<4>(b.pp));
+        kernel<<<dim3((unsigned)b.ntargets * nrhs, b.chunks), 32 * W, smem, s>>>(a, mt, b, mma::unit_size(b.pp), nrhs, ld,
+                                                                                 per_rhs);
+    });
+}
+
+void launch_translate_mma(const TransArgs& a, const MmaTabs& mt, int pp, int ntargets, int chunks, cudaStream_t s) {
+    by_degree(pp, [&]<int NI, int W, int CTAS>() {
+        auto* kernel = k_translate_mma<NI, W, CTAS>;
+        const size_t smem = mma::smem_bytes<NI>(pp);
+        raise_smem_ceiling(reinterpret_cast<const void*>(kernel), smem);
+        kernel<<<dim3(ntargets, chunks), 32 * W, smem, s>>>(a, mt, pp, mma::unit_size(pp));
+    });
+    if (chunks > 1) launch_translate_sum(a, ntargets, chunks, s);
 }
 
 // The host tables of the tensor-core operator for degrees <= pmax (k_mma.cuh).
