@@ -43,9 +43,13 @@ struct Trace {
     Trace& operator=(const Trace&) = delete;
 };
 
-// The direct operator's launches with the tensor-core operator's chunks for a number of vectors, and the slabs they fill.
+// The tensor-core operator's launches for a number of vectors, one per kernel class, and the slabs they fill.
 struct MmaPlan {
-    std::vector<DirectBucket> launches;
+    struct Launch {
+        int first, count, ctas, pp;   // shares work[first .. first + count - 1]
+    };
+    std::vector<Launch> launches;
+    MmaWork* d_work = nullptr;
     SlabUse use{};
 };
 
@@ -542,6 +546,7 @@ static_assert(kBucketBounds[kNumBounds - 1] >= kMaxDegree, "every order needs a 
 // Truncation-order buckets of the spheres and the (target bucket, source bucket) launches of
 // the direct operator.  Bucket upper bounds grow in steps of 4 degrees; each launch gets enough
 // CTAs per target to fill the GPU.
+int mma_plan(foggy_handle h, int nrhs, const MmaPlan** out);
 int plan_direct(foggy_handle h) {
     const int* bounds = kBucketBounds;
     std::vector<std::vector<int>> members;
@@ -589,48 +594,94 @@ int plan_direct(foggy_handle h) {
             b.pp = std::max(bp[t], bp[s]);
             h->launches_direct.push_back(b);
         }
-    h->mma_plans.clear();
-    return FOGGY_OK;
+    // the plans of single vectors, so that no later call allocates for them
+    const MmaPlan* plan = nullptr;
+    TRY(mma_plan(h, 1, &plan));
+    return mma_plan(h, 0, &plan);
 }
 
-// The tensor-core operator's launches for nrhs vectors at a time (at most h->cmax: each has its own slabs).  The
-// slabs of one vector and source bucket bound the chunks; among them the count is taken whose waves of CTAs cost
-// least: a wave lasts as long as its CTAs' batches plus their set-up, about 0.3 of a batch.  64 spheres of order 15
-// (one wave of 256 CTAs with four batches each, where 14 chunks ran four waves of one batch): 109 -> 102 us an
-// application; 1000 lognormal spheres: 29.9 -> 27.3 ms.
-const MmaPlan& mma_plan(foggy_handle h, int nrhs) {
-    auto it = h->mma_plans.find(nrhs);
-    if (it != h->mma_plans.end()) return it->second;
-    MmaPlan p;
-    p.launches = h->launches_direct;
-    const int nb = h->nbuckets, per = std::max(1, h->cmax / nrhs);
+// The tensor-core operator's plan for nrhs vectors at a time (at most h->cmax: each has its own slabs); nrhs = 0: one
+// vector with one slab per source bucket (foggy_matvec_static).
+//
+// All (target bucket, source bucket) shares of a kernel class are one launch, largest degrees first, so that buckets of a
+// few spheres fill the GPU together, and the next class's CTAs start while the last of a class run out.  One launch a
+// share left 83 spheres with 5 right-hand sides 25 launches of 6 to 200 CTAs; 250 lognormal spheres 2.42 -> 1.74 ms an
+// application, 1000 27.3 -> 24.0 ms, 8 spheres 108 -> 76 us.  The shares' CTAs take about the
+// same number of batches B of four translations, the B that ends first, a CTA costing its batches plus 0.3 of one for
+// its set-up, larger degrees more by their square.  Slabs bound the chunks.
+int make_mma_plan(foggy_handle h, int nrhs, MmaPlan& p) {
+    const int nb = h->nbuckets, nv = std::max(1, nrhs), per = nrhs == 0 ? 1 : std::max(1, h->cmax / nv);
     p.use.nb = nb;
     p.use.per_bucket = per;
     p.use.per_rhs = nb * per;
-    for (int i = 0; i < nb * nb; ++i) {
-        DirectBucket& b = p.launches[i];
-        const int t = i / nb, s = i % nb, batches = (b.nsources + 3) / 4;
-        const double slots = 148.0 * mma_ctas_per_sm(b.pp);
+    std::vector<MmaWork> work;
+    for (int cls = 3; cls >= 0; --cls) {
+        std::vector<int> in;
+        for (int i = 0; i < nb * nb; ++i)
+            if (h->launches_direct[i].pp <= kMmaDegree && mma_class(h->launches_direct[i].pp) == cls) in.push_back(i);
+        if (in.empty()) continue;
+        std::stable_sort(in.begin(), in.end(),
+                         [&](int a, int b) { return h->launches_direct[a].pp > h->launches_direct[b].pp; });
+        const int pp = h->launches_direct[in[0]].pp;
+        const int slots = 148 * mma_ctas_per_sm(pp);
+        auto chunks_for = [&](int i, int B) {
+            const int batches = (h->launches_direct[i].nsources + 3) / 4;
+            return std::max(1, std::min({per, batches, (batches + B - 1) / B}));
+        };
         double best = 1e300;
-        for (int c = 1; c <= std::min(batches, per); ++c) {
-            const double cost = std::ceil((double)b.ntargets * nrhs * c / slots) * ((batches + c - 1) / c + 0.3);
-            if (cost < best * 0.999) {
-                best = cost;
-                b.chunks = c;
+        int bestB = 1;
+        for (int B : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 128}) {
+            double total = 0.0, longest = 0.0;
+            int64_t ctas = 0;
+            for (int i : in) {
+                const DirectBucket& b = h->launches_direct[i];
+                const int batches = (b.nsources + 3) / 4, c = chunks_for(i, B);
+                const double cost = ((batches + c - 1) / c + 0.3) * (double)b.pp * b.pp;
+                const int64_t n = (int64_t)b.ntargets * nv * c;
+                total += cost * n;
+                ctas += n;
+                longest = std::max(longest, cost);
+            }
+            // equal CTAs run in waves; unequal ones, the largest first, leave half of one at the end
+            const double t = in.size() == 1 ? std::ceil((double)ctas / slots) * longest
+                             : ctas <= slots ? longest
+                                             : total / slots + 0.5 * longest;
+            if (t < best * 0.999) {
+                best = t;
+                bestB = B;
             }
         }
-        b.slab = s * per;
-        p.use.c[t][s] = (unsigned char)b.chunks;
+        MmaPlan::Launch l{(int)work.size(), (int)in.size(), 0, pp};
+        for (int i : in) {
+            const DirectBucket& b = h->launches_direct[i];
+            const int t = i / nb, s = i % nb, c = chunks_for(i, bestB);
+            work.push_back(MmaWork{b.targets, b.sources, b.ntargets, b.nsources, s * per, c, b.pp, mma_unit_size(b.pp), l.ctas});
+            p.use.c[t][s] = (unsigned char)c;
+            l.ctas += b.ntargets * nv * c;
+        }
+        p.launches.push_back(l);
     }
     // compact bucket of each step of four orders
     int id = 0;
     for (int q = 0; q < 12; ++q) {
-        bool any = false;
-        for (int pj : h->p_s) any |= (pj - 1) / 4 == q;
         p.use.of[q] = (unsigned char)id;
-        id += any;
+        id += std::any_of(h->p_s.begin(), h->p_s.end(), [&](int pj) { return (pj - 1) / 4 == q; });
     }
-    return h->mma_plans.emplace(nrhs, std::move(p)).first->second;
+    if (work.empty()) return FOGGY_OK;
+    TRY(dalloc(h, &p.d_work, work.size()));
+    CK(h, h2d(h, p.d_work, work.data(), work.size() * sizeof(MmaWork)));
+    return FOGGY_OK;
+}
+
+int mma_plan(foggy_handle h, int nrhs, const MmaPlan** out) {
+    auto it = h->mma_plans.find(nrhs);
+    if (it == h->mma_plans.end()) {
+        MmaPlan p;
+        TRY(make_mma_plan(h, nrhs, p));
+        it = h->mma_plans.emplace(nrhs, std::move(p)).first;
+    }
+    *out = &it->second;
+    return FOGGY_OK;
 }
 
 // The pair tables over groups of pairs (k_pair_tables.cu).  The pairs are grouped by
@@ -1378,13 +1429,21 @@ int apply_operator_fmm(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false
     return FOGGY_OK;
 }
 
-// Y_r = A X_r on the tensor cores for the nrhs <= h->cmax vectors X + r n_unk
-void launch_mma(foggy_handle h, DirectArgs a, int nrhs, const cplx* X, cplx* Y) {
-    const MmaPlan& p = mma_plan(h, nrhs);
+// Y_r = A X_r on the tensor cores for the nrhs <= h->cmax vectors X + r n_unk (nrhs = 0: foggy_matvec_static's one);
+// a.partial holds the plan's slabs
+int launch_mma(foggy_handle h, DirectArgs a, int nrhs, const cplx* X, cplx* Y) {
+    const MmaPlan* p = nullptr;
+    TRY(mma_plan(h, nrhs, &p));
     const MmaTabs mt = mma_tabs(h);
+    const int nv = std::max(1, nrhs);
     a.x = X;
-    for (const DirectBucket& b : p.launches) launch_direct_mma(a, mt, b, nrhs, h->n_unk, p.use.per_rhs, h->stream);
-    k_direct_finish<<<dim3(h->N, nrhs), 256, 0, h->stream>>>(a.sc, X, h->d_partial, p.use, h->n_unk, h->n_unk, Y);
+    for (const MmaPlan::Launch& l : p->launches)
+        launch_direct_mma(a, mt, p->d_work + l.first, l.count, l.ctas, l.pp, nv, h->n_unk, p->use.per_rhs,
+                          &l != &p->launches.front(), h->stream);
+    k_direct_finish<<<dim3(h->N, nv), 256, 0, h->stream>>>(a.sc, X, a.partial, p->use, h->n_unk, h->n_unk, Y);
+    h->launches += (int64_t)p->launches.size() + 1;
+    CKL(h);
+    return FOGGY_OK;
 }
 
 // y = A x in the device layout
@@ -1397,15 +1456,15 @@ int apply_operator(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false) {
     a.fp32 = (!mma && fp32 && h->stab32_ready) ? 1 : 0;
     Trace tr(a.fp32 ? "operator (FP32)" : "operator (FP64)");
     if (mma) {
-        launch_mma(h, a, 1, x, y);
+        TRY(launch_mma(h, a, 1, x, y));
     } else {
         for (const DirectBucket& b : h->launches_direct) launch_direct(a, b, h->stream);
         CKL(h);
         SlabUse all{};
         all.per_rhs = h->nbuckets * h->cmax;
         k_direct_finish<<<h->N, 256, 0, h->stream>>>(a.sc, x, h->d_partial, all, h->n_unk, 0, y);
+        h->launches += (int64_t)h->launches_direct.size() + 1;
     }
-    h->launches += (int64_t)h->launches_direct.size() + 1;
     CKL(h);
     return FOGGY_OK;
 }
@@ -1476,6 +1535,8 @@ void free_scene(foggy_handle h) {
     dfree(h, h->d_b);
     dfree(h, h->d_pq);
     dfree(h, h->d_partial);
+    for (auto& [nrhs, p] : h->mma_plans) dfree(h, p.d_work);
+    h->mma_plans.clear();
     dfree(h, h->d_stab);
     dfree(h, h->d_stab32);
     h->stab32_ready = false;
@@ -2702,17 +2763,20 @@ extern "C" int32_t foggy_matvec_static(foggy_handle h, const double* x, double* 
     DirectArgs a = direct_args(h, xin);
     a.partial = partial;
     a.cmax = 1;
-    for (const DirectBucket& b : h->launches_direct) {
-        DirectBucket b1 = b;
-        b1.chunks = 1;
-        b1.slab = b.slab / h->cmax;
-        if (mma_operator(h, a)) launch_direct_mma(a, mma_tabs(h), b1, 1, 0, h->nbuckets, h->stream);
-        else launch_direct(a, b1, h->stream);
+    if (mma_operator(h, a)) {
+        TRY(launch_mma(h, a, 0, xin, yout));
+    } else {
+        for (const DirectBucket& b : h->launches_direct) {
+            DirectBucket b1 = b;
+            b1.chunks = 1;
+            b1.slab = b.slab / h->cmax;
+            launch_direct(a, b1, h->stream);
+        }
+        CKL(h);
+        SlabUse all{};
+        all.per_rhs = h->nbuckets;
+        k_direct_finish<<<h->N, 256, 0, h->stream>>>(sv, xin, partial, all, h->n_unk, 0, yout);
     }
-    CKL(h);
-    SlabUse all{};
-    all.per_rhs = h->nbuckets;
-    k_direct_finish<<<h->N, 256, 0, h->stream>>>(sv, xin, partial, all, h->n_unk, 0, yout);
     k_pack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, yout, xr, reinterpret_cast<cplx*>(y));
     CKL(h);
     CK(h, cudaStreamSynchronize(h->stream));
@@ -2843,8 +2907,7 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
         Trace tr("block operator (FP64)");
         for (int r = 0; r < nrhs; r += h->cmax) {
             const int nr = std::min(h->cmax, nrhs - r);
-            launch_mma(h, ba.d, nr, X + (size_t)r * h->n_unk, Y + (size_t)r * h->n_unk);
-            h->launches += (int64_t)h->launches_direct.size() + 1;
+            TRY(launch_mma(h, ba.d, nr, X + (size_t)r * h->n_unk, Y + (size_t)r * h->n_unk));
         }
         CKL(h);
         return FOGGY_OK;

@@ -146,10 +146,23 @@ void build_mma_tables(int pmax, const std::vector<double>& delta, std::vector<do
                       std::vector<int>& plan);
 // CTAs of a launch of largest degree pp that an SM holds at once
 int mma_ctas_per_sm(int pp);
-// b.pp <= kMmaDegree, a.pt.stab set; for each of nrhs vectors (a.x + r ld) fills slabs b.slab .. b.slab + b.chunks - 1
-// of the r-th run of per_rhs slabs
-void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, int nrhs, int64_t ld, int per_rhs,
-                       cudaStream_t s);
+// the kernel instantiation of a largest degree, 0..3: launches of one class go as one
+int mma_class(int pp);
+// A (target bucket, source bucket) share of a launch: CTAs cta0 .. cta0 + ntargets nrhs chunks - 1, vector fastest, then
+// target, then chunk
+struct MmaWork {
+    const int* targets;
+    const int* sources;
+    int ntargets, nsources;
+    int slab, chunks;          // fills slabs slab .. slab + chunks - 1 of each vector's run of per_rhs
+    int pp, us;                // largest degree (<= kMmaDegree) and the shared-memory stride of a unit (mma_unit_size)
+    int cta0;
+};
+int mma_unit_size(int pp);
+// nw shares of one class, largest degree pp, `ctas` CTAs in all; a.pt.stab set, vectors a.x + r ld.  after_other: the
+// launch before it on the stream is one of these with the same input, and may still be running out
+void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const MmaWork* w, int nw, int ctas, int pp, int nrhs,
+                       int64_t ld, int per_rhs, bool after_other, cudaStream_t s);
 
 // k_pair_tables.cu -- the pair tables over groups of pairs with one M2 = max order + 2: FP32 as
 // tensor-core products (tcgen05 kind::tf32, 3xTF32; the group's pairs share the Gaunt operand, a

@@ -1494,7 +1494,16 @@ __global__ void k_direct_finish(SceneView sc, const cplx* x, const cplx* partial
             for (int b = 0; b < (use.nb ? use.nb : 1); ++b) {
                 const cplx* q = partial + (size_t)b * use.per_bucket * n_unk + o + t;
                 const int m = use.nb ? use.c[row][b] : use.per_rhs;
-                for (int c = 0; c < m; ++c) sum = sum + q[(size_t)c * n_unk];
+                int c = 0;
+                for (; c + 4 <= m; c += 4) {   // four loads in flight, added in order
+                    const cplx q0 = q[(size_t)c * n_unk], q1 = q[(size_t)(c + 1) * n_unk],
+                               q2 = q[(size_t)(c + 2) * n_unk], q3 = q[(size_t)(c + 3) * n_unk];
+                    sum = sum + q0;
+                    sum = sum + q1;
+                    sum = sum + q2;
+                    sum = sum + q3;
+                }
+                for (; c < m; ++c) sum = sum + q[(size_t)c * n_unk];
             }
             int tt = t < Pj ? t : t - Pj;
             int n, m;

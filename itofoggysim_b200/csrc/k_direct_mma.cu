@@ -129,16 +129,29 @@ __device__ __forceinline__ int batches_of(int n, int c, int chunks) {
 }  // namespace
 
 template <int NI, int W, int CTAS>
-__global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTabs mt, DirectBucket bk, int us, int nrhs,
-                                                             int64_t ld, int per_rhs) {
+__global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTabs mt, const MmaWork* __restrict__ work,
+                                                             int nw, int nrhs, int64_t ld, int per_rhs) {
     extern __shared__ __align__(16) double smem_d[];
+    // the next class's CTAs may start once all of these have (they fill other slabs); each launch ends after the one before
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const SceneView& sc = a.sc;
+    // this CTA's share: the last one that starts no later (every warp looks, one load per lane and 32 shares)
+    int at = -1;
+    for (int b = 0; b < nw; b += 32) {
+        const int i = b + (threadIdx.x & 31);
+        at += __popc(__ballot_sync(0xffffffffu, i < nw && work[i].cta0 <= (int)blockIdx.x));
+    }
+    const MmaWork bk = work[at];
     // right-hand side fastest: the CTAs that read one pair's coaxial block run together
-    const int rhs = blockIdx.x % nrhs, j = bk.targets[blockIdx.x / nrhs];
-    if (!sc.couple[j]) return;
+    const int id = blockIdx.x - bk.cta0, rhs = id % nrhs, tc = id / nrhs, c = tc / bk.ntargets;
+    const int j = bk.targets[tc % bk.ntargets];
+    if (!sc.couple[j]) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        return;
+    }
     const cplx* const x = a.x + rhs * ld;
-    const int c = blockIdx.y, pj = sc.p[j];
-    const Shared s = carve<NI>(smem_d, bk.pp, us);
+    const int pj = sc.p[j];
+    const Shared s = carve<NI>(smem_d, bk.pp, bk.us);
     run_batches<NI, W>(s, mt, bk.pp, pj, batches_of(bk.nsources, c, bk.chunks), [&](int r, Unit& un, Dir& d) {
         const int i = kUnits * (c + r / kUnits * bk.chunks) + r % kUnits;
         const int l = i < bk.nsources ? bk.sources[i] : j;
@@ -150,6 +163,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTa
     });
     cplx* out = a.partial + ((size_t)rhs * per_rhs + bk.slab + c) * a.n_unk + sc.off[j];
     for (int t = threadIdx.x; t < 2 * pj * (pj + 2); t += 32 * W) out[t] = mk(s.acc[t].x, s.acc[t].y);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // One ML-FMM pass over cached blocks (k_translate's arguments and results)
@@ -178,6 +192,8 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_translate_mma(TransArgs a, Mma
 }
 
 int mma_ctas_per_sm(int pp) { return pp <= 7 ? 4 : pp <= 23 ? 2 : 1; }
+int mma_class(int pp) { return pp <= 7 ? 0 : pp <= 15 ? 1 : pp <= 23 ? 2 : 3; }
+int mma_unit_size(int pp) { return mma::unit_size(pp); }
 
 // f(kernel tag) with the instantiation of a launch of largest degree pp
 template <class F>
@@ -188,14 +204,23 @@ static void by_degree(int pp, F f) {
     else f.template operator()<4, mma::warps_of(31), 1>();
 }
 
-void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const DirectBucket& b, int nrhs, int64_t ld, int per_rhs,
-                       cudaStream_t s) {
-    by_degree(b.pp, [&]<int NI, int W, int CTAS>() {
+void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const MmaWork* w, int nw, int ctas, int pp, int nrhs,
+                       int64_t ld, int per_rhs, bool after_other, cudaStream_t s) {
+    by_degree(pp, [&]<int NI, int W, int CTAS>() {
         auto* kernel = k_direct_mma<NI, W, CTAS>;
-        const size_t smem = mma::smem_bytes<NI>(b.pp);
+        const size_t smem = mma::smem_bytes<NI>(pp);
         raise_smem_ceiling(reinterpret_cast<const void*>(kernel), smem);
-        kernel<<<dim3((unsigned)b.ntargets * nrhs, b.chunks), 32 * W, smem, s>>>(a, mt, b, mma::unit_size(b.pp), nrhs, ld,
-                                                                                 per_rhs);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)ctas);
+        cfg.blockDim = dim3(32 * W);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = after_other ? 1 : 0;
+        cudaLaunchKernelEx(&cfg, kernel, a, mt, w, nw, nrhs, ld, per_rhs);
     });
 }
 
