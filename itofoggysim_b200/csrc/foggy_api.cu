@@ -740,7 +740,14 @@ int build_pair_tables(foggy_handle h, const SGaunt& g, bool fp64, bool fp32) {
     };
     std::vector<TcTile> t64, t32;
     std::vector<int> t64_0, t32_0;
-    if (fp64) make_tiles(false, 16, t64, t64_0);
+    if (fp64) {
+        // runs of 16 row tiles share a tile's radial functions; a small scene takes shorter ones, for four CTAs an SM
+        // (64 spheres of order 15: 63 CTAs, 325 us; 252 CTAs, 104 us)
+        int64_t ctas = 0;
+        for (size_t i = 0; i < groups.size(); ++i)
+            ctas += (gend[i] - gbeg[i] + kPairs64 - 1) / kPairs64 * ((groups[i].mtiles + 15) / 16);
+        make_tiles(false, (int)std::max<int64_t>(2, std::min<int64_t>(16, 16 * ctas / (4 * 148))), t64, t64_0);
+    }
     if (fp32) make_tiles(true, 8, t32, t32_0);
     int2* d_pairs = nullptr;
     TcTile* d_t64 = nullptr;
@@ -772,8 +779,10 @@ int build_pair_tables(foggy_handle h, const SGaunt& g, bool fp64, bool fp32) {
     if (e != cudaSuccess) return fin(fail(h, FOGGY_ERR_CUDA, std::string("pair tables: ") + cudaGetErrorString(e)));
     if (fp64) {
         PairArgs pa{scene_view(h), h->prm.z_coupling, d_pairs, d_t64, d_groups, g, h->d_pair_off, h->d_stab};
-        for (size_t i = 0; i < groups.size(); ++i) {
-            launch_pair_s_group(pa, t64_0[i], t64_0[i + 1] - t64_0[i], groups[i].M2, h->stream);
+        // the groups of one kernel instantiation (M2 up to 16, 32, 48) in one launch
+        for (size_t i = 0, e = 0; i < groups.size(); i = e) {
+            while (e < groups.size() && (groups[e].M2 - 1) / 16 == (groups[i].M2 - 1) / 16) ++e;
+            launch_pair_s_group(pa, t64_0[i], t64_0[e] - t64_0[i], groups[e - 1].M2, h->stream);
             h->launches += 1;
         }
     }

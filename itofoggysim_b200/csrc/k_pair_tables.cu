@@ -356,7 +356,9 @@ __global__ void __launch_bounds__(256) k_pair_s_group(PairArgs a, int tile0) {
     const int M2 = a.groups[tl.group].M2, P = 2 * M2 - 2, km = M2 - 2;
     cplx* zeta = reinterpret_cast<cplx*>(ps_smem);                              // [kPairs64][P + 1]
     double* scr = reinterpret_cast<double*>(zeta + (size_t)kPairs64 * (P + 1));  // [kPairs64][2 (P + 1)]
-    for (int i = tid; i < tl.count; i += 256) {
+    // the two radial sequences of a pair on threads of two warps
+    if (tid < 2 * kPairs64 && tid % kPairs64 < tl.count) {
+        const int i = tid % kPairs64;
         const int2 st = a.pairs[tl.first + i];
         const double* cs = a.sc.centres + 3 * (size_t)st.x;
         const double* ct = a.sc.centres + 3 * (size_t)st.y;
@@ -365,10 +367,13 @@ __global__ void __launch_bounds__(256) k_pair_s_group(PairArgs a, int tile0) {
         double d2 = a.sc.k * (ct[2] - cs[2]);
         const double rho = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
         double* jb = scr + (size_t)2 * (P + 1) * i;
-        dev_sph_jn(rho, P, jb);
-        if (a.z != 1) dev_sph_yn(rho, P, jb + P + 1);
-        s_off[i] = a.pair_off[pair_index(st.x, st.y, a.sc.n)];
-        s_tot[i] = pair_block_size(a.sc.p[st.x], a.sc.p[st.y]);
+        if (tid < kPairs64) {
+            dev_sph_jn(rho, P, jb);
+            s_off[i] = a.pair_off[pair_index(st.x, st.y, a.sc.n)];
+            s_tot[i] = pair_block_size(a.sc.p[st.x], a.sc.p[st.y]);
+        } else if (a.z != 1) {
+            dev_sph_yn(rho, P, jb + P + 1);
+        }
     }
     __syncthreads();
     for (int idx = tid; idx < tl.count * (P + 1); idx += 256) {
