@@ -600,7 +600,7 @@ int plan_direct(foggy_handle h) {
     return mma_plan(h, 0, &plan);
 }
 
-// The tensor-core operator's plan for nrhs vectors at a time (at most h->cmax: each has its own slabs); nrhs = 0: one
+// The tensor-core operator's plan for nrhs vectors at a time (each has its own slabs); nrhs = 0: one
 // vector with one slab per source bucket (foggy_matvec_static).
 //
 // All (target bucket, source bucket) shares of a kernel class are one launch, largest degrees first, so that buckets of a
@@ -1438,8 +1438,8 @@ int apply_operator_fmm(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false
     return FOGGY_OK;
 }
 
-// Y_r = A X_r on the tensor cores for the nrhs <= h->cmax vectors X + r n_unk (nrhs = 0: foggy_matvec_static's one);
-// a.partial holds the plan's slabs
+// Y_r = A X_r on the tensor cores for the nrhs vectors X + r n_unk (nrhs = 0: foggy_matvec_static's one); a.partial
+// holds the plan's slabs
 int launch_mma(foggy_handle h, DirectArgs a, int nrhs, const cplx* X, cplx* Y) {
     const MmaPlan* p = nullptr;
     TRY(mma_plan(h, nrhs, &p));
@@ -1595,7 +1595,10 @@ int ensure_workspace(foggy_handle h, int restart) {
     TRY(dalloc(h, &h->d_part, (size_t)kRedBlocks * (restart + 1)));
     if (!h->d_npart) TRY(dalloc(h, &h->d_npart, kRedBlocks));
     if (!h->d_scal) TRY(dalloc(h, &h->d_scal, 8));
-    if (!h->d_flags) TRY(dalloc(h, &h->d_flags, 4));
+    if (!h->d_flags) {
+        TRY(dalloc(h, &h->d_flags, 4));   // flags, ticket
+        CK(h, cudaMemsetAsync(h->d_flags, 0, 4 * sizeof(int), h->stream));
+    }
     h->ws_restart = restart;
     return FOGGY_OK;
 }
@@ -1685,18 +1688,28 @@ int gmres(foggy_handle h, foggy_stats* st) {
             cplx* vk = h->d_V + (size_t)k * n;
             cplx* vk1 = h->d_V + (size_t)(k + 1) * n;
             TRY(matvec(vk, h->d_w, true));
-            k_dots_partial<<<kRedBlocks, 256, 0, h->stream>>>(h->d_V, n, k + 1, h->d_w, n, h->d_part);
-            k_dots_reduce<<<k + 1, 256, 0, h->stream>>>(h->d_part, k + 1, h->d_h, 0);
-            k_axpy_multi<<<G, 256, 0, h->stream>>>(h->d_V, n, k + 1, h->d_h, h->d_w, n);
-            k_dots_partial<<<kRedBlocks, 256, 0, h->stream>>>(h->d_V, n, k + 1, h->d_w, n, h->d_part);
-            k_dots_reduce<<<k + 1, 256, 0, h->stream>>>(h->d_part, k + 1, h->d_c, 0);
-            k_axpy_multi<<<G, 256, 0, h->stream>>>(h->d_V, n, k + 1, h->d_c, h->d_w, n);
-            TRY(norm_dev(h, h->d_w, d_hn));
-            k_scale_copy<<<G, 256, 0, h->stream>>>(h->d_w, d_hn, vk1, n);
-            k_givens<<<1, 1, 0, h->stream>>>(h->d_H, m, h->d_cs, h->d_sn, h->d_gv, h->d_h, h->d_c, d_hn, k, d_res,
-                                             h->d_flags);
+            GsArgs gs{};
+            gs.V = h->d_V;
+            gs.ldi = n;
+            gs.nv = k + 1;
+            gs.m = m;
+            gs.W = h->d_w;
+            gs.n = n;
+            gs.part = h->d_part;
+            gs.hh = h->d_h;
+            gs.c = h->d_c;
+            gs.H = h->d_H;
+            gs.cs = h->d_cs;
+            gs.g = h->d_gv;
+            gs.npart = h->d_npart;
+            gs.hn = d_hn;
+            gs.sn = h->d_sn;
+            gs.res = d_res;
+            gs.flags = h->d_flags;
+            gs.ticket = h->d_flags + 1;
+            launch_arnoldi_step(gs, 1, vk1, h->stream);
             CKL(h);
-            h->launches += 8;
+            h->launches += 4;
             const int sl = k & 1;
             CK(h, cudaMemcpyAsync(h->h_pin + 4 * sl, h->d_scal, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
             CK(h, cudaMemcpyAsync(h->h_pin_flags + sl, h->d_flags, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -2949,7 +2962,8 @@ int ensure_block_ws(foggy_handle h, int nrhs, int m) {
     TRY(dalloc(h, &h->d_bsmall, nb * ((size_t)(m + 1) * m + m + 4 * (size_t)(m + 1) + (size_t)(m + 1) * kRedBlocks)));
     // sn m, bnorm, beta, hn, tol, res per slot; norm partials kRedBlocks per slot
     TRY(dalloc(h, &h->d_breal, nb * ((size_t)m + 5 + kRedBlocks)));
-    TRY(dalloc(h, &h->d_bint, 3 * nb));
+    TRY(dalloc(h, &h->d_bint, 4 * nb));
+    CK(h, cudaMemsetAsync(h->d_bint, 0, 4 * nb * sizeof(int), h->stream));
     h->blk_nrhs = nrhs;
     h->blk_m = m;
     return FOGGY_OK;
@@ -2958,7 +2972,7 @@ int ensure_block_ws(foggy_handle h, int nrhs, int m) {
 struct BlockPtrs {
     cplx *H, *cs, *g, *hh, *c, *y, *part;
     double *sn, *bnorm, *beta, *hn, *tol, *res, *npart;
-    int *live, *kend, *flags;
+    int *live, *kend, *flags, *ticket;
 };
 
 BlockPtrs block_ptrs(foggy_handle h) {
@@ -2983,6 +2997,7 @@ BlockPtrs block_ptrs(foggy_handle h) {
     p.live = h->d_bint;
     p.kend = h->d_bint + nb;
     p.flags = h->d_bint + 2 * nb;
+    p.ticket = h->d_bint + 3 * nb;
     return p;
 }
 
@@ -3094,19 +3109,31 @@ int block_gmres(foggy_handle h, int nrhs, foggy_stats* st, std::vector<int>& ite
             cplx* Vk1 = h->d_bV + (size_t)(k + 1) * ldi;
             rc = matvec(Vk, h->d_bW, nact, true);
             if (rc) { done(); return rc; }
-            for (int pass = 0; pass < 2; ++pass) {
-                cplx* coef = pass ? p.c : p.hh;
-                k_dots_partial_b<<<dim3(kRedBlocks, nact), 256, 0, h->stream>>>(h->d_bV, ldi, n, k + 1, h->d_bW, n,
-                                                                                p.live, p.part);
-                k_dots_reduce_b<<<dim3(k + 1, nact), 256, 0, h->stream>>>(p.part, k + 1, p.live, coef, m + 1);
-                k_axpy_multi_b<<<dim3(G, nact), 256, 0, h->stream>>>(h->d_bV, ldi, n, k + 1, coef, m + 1, h->d_bW, n,
-                                                                     p.live);
-            }
-            TRY(block_norms(h, h->d_bW, nact, p.live, p.hn, p));
-            k_scale_copy_b<<<dim3(G, nact), 256, 0, h->stream>>>(h->d_bW, n, p.hn, 1, Vk1, n, n, p.live);
-            k_givens_b<<<(nact + 63) / 64, 64, 0, h->stream>>>(p.H, m, p.cs, p.sn, p.g, p.hh, p.c, p.hn, k, p.tol,
-                                                                p.res, p.flags, p.live, p.kend, nact);
-            h->launches += 8;
+            GsArgs gs{};
+            gs.V = h->d_bV;
+            gs.ldi = ldi;
+            gs.ld = n;
+            gs.nv = k + 1;
+            gs.m = m;
+            gs.W = h->d_bW;
+            gs.n = n;
+            gs.part = p.part;
+            gs.hh = p.hh;
+            gs.c = p.c;
+            gs.H = p.H;
+            gs.cs = p.cs;
+            gs.g = p.g;
+            gs.npart = p.npart;
+            gs.hn = p.hn;
+            gs.sn = p.sn;
+            gs.res = p.res;
+            gs.tol = p.tol;
+            gs.flags = p.flags;
+            gs.live = p.live;
+            gs.kend = p.kend;
+            gs.ticket = p.ticket;
+            launch_arnoldi_step(gs, nact, Vk1, h->stream);
+            h->launches += 4;
             CKL(h);
             // slots live at this step did an Arnoldi step
             std::vector<int> was(hlive.begin(), hlive.begin() + nact);

@@ -268,34 +268,38 @@ __global__ void k_translation_pair(AxialView ax, DTabs dt, double x, double thet
 
 // k_gmres.cu -- Krylov kernels (deterministic fixed-order reductions)
 constexpr int kRedBlocks = 296;
-__global__ void k_dots_partial(const cplx* V, int64_t ld, int nv, const cplx* w, int64_t n, cplx* part);
-__global__ void k_dots_reduce(const cplx* part, int nv, cplx* out, int accumulate);
-__global__ void k_axpy_multi(const cplx* V, int64_t ld, int nv, const cplx* h, cplx* w, int64_t n);
+// Orthogonalisation of one Arnoldi step (classical Gram-Schmidt twice, norm, Givens rotation) for one Krylov space, or one
+// per slot: basis vector i of slot b at V + i ldi + b ld, nv = k + 1 of them, the new vector at W + b ld.  Per slot: hh, c,
+// g (m + 1 entries), H ((m + 1) x m, row-major), cs, sn (m), hn, res, flags, ticket (0 between launches), part
+// (nv x kRedBlocks), npart (kRedBlocks).  live (null: all), kend and tol are the slots' state in a block solve.
+struct GsArgs {
+    const cplx* V;
+    int64_t ldi, ld;
+    int nv, m;
+    cplx* W;
+    int64_t n;
+    cplx *part, *hh, *c, *H, *cs, *g;
+    double *npart, *hn, *sn, *res;
+    const double* tol;
+    int *flags, *live, *kend, *ticket;
+};
+// the step's launches; the normalised vector goes to Vnext + b ld
+void launch_arnoldi_step(const GsArgs& a, int slots, cplx* Vnext, cudaStream_t s);
 __global__ void k_norm_partial(const cplx* w, int64_t n, double* part);
 __global__ void k_norm_reduce(const double* part, double* out);
 __global__ void k_scale_copy(const cplx* w, const double* nrm, cplx* v, int64_t n);
 __global__ void k_sub(const cplx* b, const cplx* ax, cplx* r, int64_t n);
-__global__ void k_givens(cplx* H, int ldh, cplx* cs, double* sn, cplx* g, const cplx* h, const cplx* c,
-                         const double* hn, int k, double* res_est, int* flags);
 __global__ void k_trisolve(const cplx* H, int ldh, const cplx* g, int k, cplx* y);
 __global__ void k_update_x(cplx* x, const cplx* V, int64_t ld, const cplx* y, int k, int64_t n);
 __global__ void k_init_cycle(cplx* g, int m1, const double* beta, int* flags);
 // several right-hand sides: one Krylov space per slot (blockIdx.y), basis vector i of slot b at
 // V + i ldi + b ld; live[b] = 0 skips a slot that has left the restart cycle
-__global__ void k_dots_partial_b(const cplx* V, int64_t ldi, int64_t ld, int nv, const cplx* W, int64_t n,
-                                 const int* live, cplx* part);
-__global__ void k_dots_reduce_b(const cplx* part, int nv, const int* live, cplx* out, int ostride);
-__global__ void k_axpy_multi_b(const cplx* V, int64_t ldi, int64_t ld, int nv, const cplx* h, int hstride, cplx* W,
-                               int64_t n, const int* live);
 __global__ void k_norm_partial_b(const cplx* W, int64_t ld, int64_t n, const int* live, double* part);
 __global__ void k_norm_reduce_b(const double* part, const int* live, double* out, int ostride);
 __global__ void k_scale_copy_b(const cplx* W, int64_t ldw, const double* nrm, int nstride, cplx* Vout, int64_t ldv,
                                int64_t n, const int* live);
 __global__ void k_sub_b(const cplx* Bv, const cplx* AX, cplx* Rv, int64_t ld, int64_t n);
 __global__ void k_init_cycle_b(cplx* g, int m1, const double* beta, int nslots, int* live, int* kend);
-__global__ void k_givens_b(cplx* H, int m, cplx* cs, double* sn, cplx* g, const cplx* h, const cplx* c,
-                           const double* hn, int k, const double* tol_abs, double* res_est, int* flags, int* live,
-                           int* kend, int nslots);
 __global__ void k_trisolve_b(const cplx* H, int m, const cplx* g, const int* kend, cplx* y, int nslots);
 __global__ void k_update_x_b(cplx* X, int64_t ld, const cplx* V, int64_t ldi, const cplx* y, int ystride,
                              const int* kend, int64_t n);
