@@ -191,6 +191,8 @@ struct foggy_handle_s {
     // several right-hand sides in one block (foggy_solve_block, foggy_matvec_block): vectors of
     // nrhs slots, n_unk entries apart
     int blk_nrhs = 0, blk_m = 0;
+    cplx* d_bslab = nullptr;         // operator slabs of bslab_vectors vectors, one per source bucket
+    int bslab_vectors = 0;
     cplx* d_bV = nullptr;            // Krylov basis: vector i of slot b at (i nrhs + b) n_unk
     cplx* d_bW = nullptr;            // operator output
     cplx* d_bX = nullptr;            // iterates, slot order
@@ -1544,6 +1546,8 @@ void free_scene(foggy_handle h) {
     dfree(h, h->d_b);
     dfree(h, h->d_pq);
     dfree(h, h->d_partial);
+    dfree(h, h->d_bslab);
+    h->bslab_vectors = 0;
     for (auto& [nrhs, p] : h->mma_plans) dfree(h, p.d_work);
     h->mma_plans.clear();
     dfree(h, h->d_stab);
@@ -2817,6 +2821,7 @@ namespace {
 
 // Tile width R per launch shape, chosen by timing: (FP32, pair tables, largest degree, log2 of the
 // target count, block width up to 8) -> R.  Process-wide, as the choice depends on the shape only.
+constexpr size_t kBlockSlabBytes = (size_t)128 << 20;   // slabs of many vectors at once on the tensor cores
 std::mutex g_tile_mu;
 std::map<std::tuple<int, int, int, int, int>, int> g_tile_cache;
 
@@ -2923,13 +2928,30 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
     TRY(ensure_pair_tables(h, must32));
     const BlockArgs ba = block_args(h, X, Y, nrhs, fp32);
     if (!must32 && mma_operator(h, ba.d)) {
-        // as many vectors at a time as have slabs.  One vector per CTA: a batch's set-up that vectors could share is
-        // small beside its products, and the pair's coaxial block comes from L2 after the first.  83 spheres, 5
-        // right-hand sides to 1e-6: 161 -> 55 ms a request (the tile autotuner's runs are gone too)
+        // One vector per CTA: a batch's set-up that vectors could share is small beside its products, and the pair's
+        // coaxial block comes from L2 after the first.  83 spheres, 5 right-hand sides to 1e-6: 161 -> 55 ms a request
+        // (the tile autotuner's runs are gone too).  As many vectors at a time as have slabs: the handle's own, or a
+        // buffer of up to kBlockSlabBytes where that holds more, so that the waves of a small scene's CTAs end
+        // together (64 spheres, 32 vectors: 14 + 14 + 4 vectors took 9 waves of 296 CTAs, 32 take 7).
         Trace tr("block operator (FP64)");
-        for (int r = 0; r < nrhs; r += h->cmax) {
-            const int nr = std::min(h->cmax, nrhs - r);
-            TRY(launch_mma(h, ba.d, nr, X + (size_t)r * h->n_unk, Y + (size_t)r * h->n_unk));
+        DirectArgs a = ba.d;
+        int most = h->cmax;
+        const size_t one = (size_t)h->nbuckets * h->n_unk;
+        const int fit = (int)std::min<size_t>(nrhs, kBlockSlabBytes / (one * sizeof(cplx)));
+        if (nrhs > most && fit > most) {
+            if (h->bslab_vectors < fit) {
+                dfree(h, h->d_bslab);
+                h->bslab_vectors = dalloc(h, &h->d_bslab, one * fit) == FOGGY_OK ? fit : 0;
+            }
+            if (h->bslab_vectors > most) {
+                most = h->bslab_vectors;
+                a.partial = h->d_bslab;
+            }
+        }
+        const int groups = (nrhs + most - 1) / most, per = (nrhs + groups - 1) / groups;
+        for (int r = 0; r < nrhs; r += per) {
+            const int nr = std::min(per, nrhs - r);
+            TRY(launch_mma(h, a, nr, X + (size_t)r * h->n_unk, Y + (size_t)r * h->n_unk));
         }
         CKL(h);
         return FOGGY_OK;
