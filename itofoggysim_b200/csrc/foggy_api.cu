@@ -516,7 +516,7 @@ MmaTabs mma_tabs(foggy_handle h) {
 // Whether the FP64 operator runs on the tensor cores: over the pair tables, orders up to kMmaDegree.  It is the
 // faster one at every order it takes (222 spheres of one order: 7 0.29 against 1.39 ms, 15 0.76 / 2.0, 23 1.83 / 4.9,
 // 31 3.7 / 9.7); without tables k_direct's seven stages sum S where they use it.
-bool mma_operator(foggy_handle h, const DirectArgs& a) { return a.pt.stab && h->pmax <= kMmaDegree; }
+bool mma_operator(foggy_handle h, const DirectArgs&) { return h->pmax <= kMmaDegree; }
 
 DirectArgs direct_args(foggy_handle h, const cplx* x) {
     DirectArgs a;
@@ -2927,7 +2927,8 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
     }
     TRY(ensure_pair_tables(h, must32));
     const BlockArgs ba = block_args(h, X, Y, nrhs, fp32);
-    if (!must32 && mma_operator(h, ba.d)) {
+    // without tables the CUDA-core kernel sums S once for a tile of vectors
+    if (!must32 && mma_operator(h, ba.d) && (ba.d.pt.stab || nrhs == 1)) {
         // One vector per CTA: a batch's set-up that vectors could share is small beside its products, and the pair's
         // coaxial block comes from L2 after the first.  83 spheres, 5 right-hand sides to 1e-6: 161 -> 55 ms a request
         // (the tile autotuner's runs are gone too).  As many vectors at a time as have slabs: the handle's own, or a
@@ -3373,7 +3374,7 @@ int32_t foggy_block_tiles(foggy_handle h, int32_t precision, int32_t nrhs, int32
         const DirectBucket& b = h->launches_direct[i];
         int R = 0;
         // one vector per CTA on the tensor cores
-        if (!ba.d.fp32 && mma_operator(h, ba.d)) R = 1;
+        if (!ba.d.fp32 && mma_operator(h, ba.d) && (tabs || nrhs == 1)) R = 1;
         else rc = choose_tile(h, ba, b, tabs, &R);
         out[4 * i] = b.ntargets;
         out[4 * i + 1] = b.nsources;

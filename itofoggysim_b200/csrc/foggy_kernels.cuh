@@ -159,7 +159,7 @@ struct MmaWork {
     int cta0;
 };
 int mma_unit_size(int pp);
-// nw shares of one class, largest degree pp, `ctas` CTAs in all; a.pt.stab set, vectors a.x + r ld.  after_other: the
+// nw shares of one class, largest degree pp, `ctas` CTAs in all; without a.pt.stab S is summed; vectors a.x + r ld.  after_other: the
 // launch before it on the stream is one of these with the same input, and may still be running out
 void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const MmaWork* w, int nw, int ctas, int pp, int nrhs,
                        int64_t ld, int per_rhs, bool after_other, cudaStream_t s);

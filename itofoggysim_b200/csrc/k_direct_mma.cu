@@ -25,8 +25,11 @@ __device__ __noinline__ Dir pair_dir_call(const double* ct, const double* cs, do
 
 // The translations of one target of degree pj, `mine` batches of four units; unit(i, l, un, dir) fills the record of unit
 // i of this CTA's batches, or leaves it empty.  The sums are in s.acc at the end, visible to every thread.
-template <int NI, int W, class UnitOf>
-__device__ __forceinline__ void run_batches(const Shared& s, const MmaTabs& mt, int pp, int pj, int mine, UnitOf unit) {
+// Without tables (SUM) the coaxial coefficients are summed from g and the radial functions of selector z; zeta: shared
+// memory for them (sum_smem_bytes).
+template <int NI, int W, bool SUM, class UnitOf>
+__device__ __forceinline__ void run_batches(const Shared& s, const MmaTabs& mt, int pp, int pj, int mine, const SGaunt& g,
+                                            int z, double2* zeta, UnitOf unit) {
     constexpr int T = 32 * W, LD = phase_ld<NI>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int Pj = pj * (pj + 2);
@@ -56,7 +59,11 @@ __device__ __forceinline__ void run_batches(const Shared& s, const MmaTabs& mt, 
             const double f = !half || m == 0 ? 1.0 : (m & 1) ? -2.0 : 2.0;
             (half ? s.eth : s.eps)[e * kUnits * LD + r] = make_double2(f * z.x, f * z.y);
         }
-        if (warp == W - 1) {
+        if constexpr (SUM) {
+            constexpr int ZL = zeta_ld<NI>();
+            if (warp == i % W)
+                radial(s.un + at, pj, z, zeta + e * kUnits * ZL, ZL, reinterpret_cast<double*>(zeta + 2 * kUnits * ZL), lane);
+        } else if (warp == W - 1) {
 #pragma unroll 1
             for (int u = 0; u < kUnits; ++u) {
                 const Unit& un = s.un[at + u];
@@ -92,7 +99,11 @@ __device__ __forceinline__ void run_batches(const Shared& s, const MmaTabs& mt, 
             rotate_all<NI>(s, L, mt.frag, warp, out ? pj : pl4, pj, mine_u, cur, out != 0);
             if (out) break;
             __syncthreads();
-            coaxial<NI>(s, un[warp % kUnits], warp % kUnits, warp / kUnits, W / kUnits, pj, mt.wf, mt.ld, lane);
+            if constexpr (SUM)
+                coaxial_sum<NI>(s, un, 2 * (warp & 1), warp / 2, W / 2, pj, mt.wf, mt.ld, g,
+                                zeta + cur * kUnits * zeta_ld<NI>(), zeta_ld<NI>(), lane);
+            else
+                coaxial<NI>(s, un[warp % kUnits], warp % kUnits, warp / kUnits, W / kUnits, pj, mt.wf, mt.ld, lane);
             if (ib + 1 < mine) {
                 prep(ib + 1, cur ^ 1);
                 // the next eight batches' records go where the last eight's were
@@ -128,7 +139,7 @@ __device__ __forceinline__ int batches_of(int n, int c, int chunks) {
 }
 }  // namespace
 
-template <int NI, int W, int CTAS>
+template <int NI, int W, int CTAS, bool SUM>
 __global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTabs mt, const MmaWork* __restrict__ work,
                                                              int nw, int nrhs, int64_t ld, int per_rhs) {
     extern __shared__ __align__(16) double smem_d[];
@@ -151,13 +162,17 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTa
     }
     const cplx* const x = a.x + rhs * ld;
     const int pj = sc.p[j];
-    const Shared s = carve<NI>(smem_d, bk.pp, bk.us);
-    run_batches<NI, W>(s, mt, bk.pp, pj, batches_of(bk.nsources, c, bk.chunks), [&](int r, Unit& un, Dir& d) {
+    // the summed variant's radial functions come first, so that the rest is laid out as ever
+    double2* const zeta = reinterpret_cast<double2*>(smem_d);
+    const Shared s = carve<NI>(SUM ? zeta + sum_smem_bytes<NI>() / 16 : zeta, bk.pp, bk.us);
+    run_batches<NI, W, SUM>(s, mt, bk.pp, pj, batches_of(bk.nsources, c, bk.chunks), a.g, a.z, zeta,
+                            [&](int r, Unit& un, Dir& d) {
         const int i = kUnits * (c + r / kUnits * bk.chunks) + r % kUnits;
         const int l = i < bk.nsources ? bk.sources[i] : j;
         if (l == j) return;
         un.x = reinterpret_cast<const double2*>(x + sc.off[l]);
-        un.s = reinterpret_cast<const double2*>(a.pt.stab + a.pt.pair_off[pair_index(min(j, l), max(j, l), sc.n)]);
+        if (!SUM)
+            un.s = reinterpret_cast<const double2*>(a.pt.stab + a.pt.pair_off[pair_index(min(j, l), max(j, l), sc.n)]);
         un.p = sc.p[l];
         d = pair_dir_call(sc.centres + 3 * (size_t)j, sc.centres + 3 * (size_t)l, sc.k, 1.0, 0.0, 0.0, 0.0);
     });
@@ -174,7 +189,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_translate_mma(TransArgs a, Mma
     const int pj = a.tgt.p[t];
     const int i0 = a.lptr[blockIdx.x], n = a.lptr[blockIdx.x + 1] - i0;
     const Shared s = carve<NI>(smem_d, pp, us);
-    run_batches<NI, W>(s, mt, pp, pj, batches_of(n, c, chunks), [&](int r, Unit& un, Dir& d) {
+    run_batches<NI, W, false>(s, mt, pp, pj, batches_of(n, c, chunks), SGaunt{}, 0, nullptr, [&](int r, Unit& un, Dir& d) {
         const int i = kUnits * (c + r / kUnits * chunks) + r % kUnits;
         if (i >= n) return;
         const int l = a.lidx[i0 + i];
@@ -207,8 +222,9 @@ static void by_degree(int pp, F f) {
 void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const MmaWork* w, int nw, int ctas, int pp, int nrhs,
                        int64_t ld, int per_rhs, bool after_other, cudaStream_t s) {
     by_degree(pp, [&]<int NI, int W, int CTAS>() {
-        auto* kernel = k_direct_mma<NI, W, CTAS>;
-        const size_t smem = mma::smem_bytes<NI>(pp);
+        const bool sum = a.pt.stab == nullptr;
+        auto* kernel = sum ? k_direct_mma<NI, W, CTAS, true> : k_direct_mma<NI, W, CTAS, false>;
+        const size_t smem = mma::smem_bytes<NI>(pp) + (sum ? mma::sum_smem_bytes<NI>() : 0);
         raise_smem_ceiling(reinterpret_cast<const void*>(kernel), smem);
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)ctas);

@@ -531,5 +531,128 @@ __device__ __forceinline__ void coaxial(const Shared& s, const Unit un, int u, i
     }
 }
 
+// ---- coaxial step without tables -----------------------------------------------------------------------
+// Radial functions of the four units of a batch, zeta_p = i^p z_p for p = 0..pj + pl + 1 and zero around them (kZetaPad
+// entries before: the sums run past an entry's own last term, where the coefficients are zero), by one warp: j_n and
+// y_n each on its own lane, then all lanes.
+constexpr int kZetaPad = 16;
+__device__ __forceinline__ void radial(const Unit* un, int pj, int z, double2* zeta, int zl, double* scratch, int lane) {
+    if (lane < 2 * kUnits) {
+        const int u = lane % kUnits, P = pj + un[u].p + 1;
+        double* o = scratch + lane * zl;
+        if (un[u].km >= 0) {
+            if (lane < kUnits) dev_sph_jn(un[u].rho, P, o);
+            else if (z != 1) dev_sph_yn(un[u].rho, P, o);
+        }
+    }
+    __syncwarp();
+    for (int t = lane; t < kUnits * zl; t += 32) {
+        const int u = t / zl, p = t - u * zl - kZetaPad;
+        cplx v = mk(0.0, 0.0);
+        if (un[u].km >= 0 && p >= 0 && p <= pj + un[u].p + 1)
+            v = zeta_of(z, p, scratch + u * zl, scratch + (kUnits + u) * zl);
+        zeta[t] = make_double2(v.x, v.y);
+    }
+}
+
+// Orders k0, k0 + dk, ... of units u0 and u0 + 1, with S(k; n, mu) = sum_q G_q(k; mu, n) zeta_{n + mu - 2q} summed for each
+// fragment entry: one Gaunt coefficient serves both units, and the tiles' accumulators stay in registers so that w is
+// formed once.  Bound by the L1's lookups for G and zeta.
+template <int NI>
+__device__ __forceinline__ void coaxial_sum(const Shared& s, const Unit* un, int u0, int k0, int dk, int pj,
+                                            const double2* __restrict__ wf, int ld, const SGaunt& g, const double2* zeta,
+                                            int zl, int lane) {
+    const int r = lane >> 2, q = lane & 3, c = r >> 1, im = r & 1;
+    const int km = max(un[u0].km, un[u0 + 1].km);
+    const int ca = 2 * c + im, cb = (2 * c + im) ^ 3, co = (2 * c + im) ^ 1;
+#pragma unroll 1
+    for (int k = k0; k <= km; k += dk) {
+        const int lo = k < 1 ? 1 : k, W = g.NM - k + 1;
+        const size_t plane = (size_t)W * W;
+        const double* G0 = g.gs + g.koff[k];
+        const double kk = (c & 2) ? -(double)k : (double)k;
+        int pl[2];
+        double rho[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const Unit& u = un[u0 + e];
+            pl[e] = k <= u.km ? u.p : -2;   // a unit without this order reads zeros
+            rho[e] = im ? u.rho : -u.rho;
+        }
+        const int top = max(pl[0], pl[1]) + 1;
+        double acc[NI][2][4];
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) acc[i][e][0] = acc[i][e][1] = acc[i][e][2] = acc[i][e][3] = 0.0;
+        double m = (double)(k + q);
+#pragma unroll 1
+        for (int mu0 = k; mu0 <= top; mu0 += 4, m += 4.0) {
+            const int mu = mu0 + q;
+            const double2 gf = __ldg(wf + k * ld + mu);
+            const double h = fma(4.0, m, 2.0), c0 = fma(m, m, m) * h;
+            double w[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const double* xd = reinterpret_cast<const double*>(s.buf + (u0 + e) * s.us + s.blk[k]);
+                const int zo = (int)(reinterpret_cast<const double*>(s.zero) - xd);
+                const int row = 8 * (mu - lo);
+                const int ra = mu >= lo && mu <= pl[e] ? row : zo, rm = mu - 1 >= lo && mu - 1 <= pl[e] ? row - 8 : zo;
+                const int rp = mu + 1 <= pl[e] ? row + 8 : zo;
+                double v = fma(gf.x, xd[rm + co], -gf.y * xd[rp + co]);
+                v = fma(kk * h, xd[ra + cb], v);
+                w[e] = fma(rho[e], v, c0 * xd[ra + ca]);
+            }
+            const int mc = min(mu, top);
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                if (lo + 8 * i > pj) break;
+                const int n = min(lo + 8 * i + r, pj);
+                const double* G = G0 + (size_t)(mc - k) * W + (n - k);
+                // past the entry's own min(n, mu) the coefficients are zero
+                const int qm = min(min(lo + 8 * i + 7, pj), min(mu0 + 3, top));
+                double sx[2] = {0.0, 0.0}, sy[2] = {0.0, 0.0};
+                const double2* z0 = zeta + u0 * zl + kZetaPad + n + mc;
+                const double2* z1 = z0 + zl;
+#pragma unroll 4
+                for (int qq = 0; qq <= qm; ++qq, z0 -= 2, z1 -= 2) {
+                    const double gq = __ldg(G);
+                    G += plane;
+                    const double2 za = *z0, zb = *z1;
+                    sx[0] = fma(gq, za.x, sx[0]);
+                    sy[0] = fma(gq, za.y, sy[0]);
+                    sx[1] = fma(gq, zb.x, sx[1]);
+                    sy[1] = fma(gq, zb.y, sy[1]);
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) mma16x8x4(acc[i][e], sx[e], sy[e], w[e]);
+            }
+        }
+        __syncwarp();
+        const int fm = k << 31;
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int n = lo + 8 * i + r;
+            if (n > pj) break;
+            const double f = flip(s.rn[n], fm);
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (pl[e] >= 0)
+                    s.buf[(u0 + e) * s.us + s.blk[k] + 4 * (n - lo) + q] =
+                        make_double2(f * (acc[i][e][0] - acc[i][e][3]), f * (acc[i][e][1] + acc[i][e][2]));
+        }
+        __syncwarp();
+    }
+}
+// entries of a unit's zeta, and the shared memory of two batches' tables and one's scratch
+template <int NI>
+__host__ __device__ constexpr int zeta_ld() {
+    return 16 * NI + 2 + kZetaPad;
+}
+template <int NI>
+__host__ __device__ constexpr size_t sum_smem_bytes() {
+    return (size_t)kUnits * zeta_ld<NI>() * (2 * 16 + 2 * 8);
+}
+
 }  // namespace mma
 }  // namespace foggy
