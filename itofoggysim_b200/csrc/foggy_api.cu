@@ -115,7 +115,7 @@ struct foggy_handle_s {
     int K = 0;
     // operator launches: (target bucket, source bucket) pairs of truncation-order buckets
     std::vector<DirectBucket> launches_direct;
-    std::map<int, MmaPlan> mma_plans;   // the tensor-core operator's launches by number of vectors
+    std::map<std::pair<int, bool>, MmaPlan> mma_plans;   // the tensor-core operator's, by vectors and no tables
     int* d_bucket_lists = nullptr;
     int nbuckets = 0, cmax = 1;
     // waves and right-hand side
@@ -540,15 +540,17 @@ DirectArgs direct_args(foggy_handle h, const cplx* x) {
 }
 
 // Upper bounds of the truncation-order buckets: steps of 4 degrees up to the largest order a
-// sphere may have (kMaxDegree, the reference's cap), so every sphere is in one bucket.
-constexpr int kBucketBounds[] = {0, 4, 8, 12, 16, 20, 24, 28, 32, 36, 40, 44, 48};
+// sphere may have (kMaxDegree, the reference's cap), so every sphere is in one bucket.  They end where the
+// tensor-core kernel's classes do (orders 7, 15, 23, 31): with bounds at 4, 8, 12, ... the orders 13..16 and 21..24 ran
+// in the class above for the sake of the last of them.
+constexpr int kBucketBounds[] = {0, 3, 7, 11, 15, 19, 23, 27, 31, 35, 39, 43, 47};
 constexpr int kNumBounds = (int)(sizeof(kBucketBounds) / sizeof(kBucketBounds[0]));
 static_assert(kBucketBounds[kNumBounds - 1] >= kMaxDegree, "every order needs a bucket");
 
 // Truncation-order buckets of the spheres and the (target bucket, source bucket) launches of
 // the direct operator.  Bucket upper bounds grow in steps of 4 degrees; each launch gets enough
 // CTAs per target to fill the GPU.
-int mma_plan(foggy_handle h, int nrhs, const MmaPlan** out);
+int mma_plan(foggy_handle h, int nrhs, bool sum, const MmaPlan** out);
 int plan_direct(foggy_handle h) {
     const int* bounds = kBucketBounds;
     std::vector<std::vector<int>> members;
@@ -598,11 +600,11 @@ int plan_direct(foggy_handle h) {
         }
     // the plans of single vectors, so that no later call allocates for them
     const MmaPlan* plan = nullptr;
-    TRY(mma_plan(h, 1, &plan));
-    return mma_plan(h, 0, &plan);
+    for (int i = 0; i < 4; ++i) TRY(mma_plan(h, i & 1, (i & 2) != 0, &plan));
+    return FOGGY_OK;
 }
 
-// The tensor-core operator's plan for nrhs vectors at a time (each has its own slabs); nrhs = 0: one
+// The tensor-core operator's plan for nrhs vectors at a time (each has its own slabs), over the pair tables or summing S (sum); nrhs = 0: one
 // vector with one slab per source bucket (foggy_matvec_static).
 //
 // All (target bucket, source bucket) shares of a kernel class are one launch, largest degrees first, so that buckets of a
@@ -611,21 +613,21 @@ int plan_direct(foggy_handle h) {
 // application, 1000 27.3 -> 24.0 ms, 8 spheres 108 -> 76 us.  The shares' CTAs take about the
 // same number of batches B of four translations, the B that ends first, a CTA costing its batches plus 0.3 of one for
 // its set-up, larger degrees more by their square.  Slabs bound the chunks.
-int make_mma_plan(foggy_handle h, int nrhs, MmaPlan& p) {
+int make_mma_plan(foggy_handle h, int nrhs, bool sum, MmaPlan& p) {
     const int nb = h->nbuckets, nv = std::max(1, nrhs), per = nrhs == 0 ? 1 : std::max(1, h->cmax / nv);
     p.use.nb = nb;
     p.use.per_bucket = per;
     p.use.per_rhs = nb * per;
     std::vector<MmaWork> work;
-    for (int cls = 3; cls >= 0; --cls) {
+    for (int cls = 4; cls >= 0; --cls) {
         std::vector<int> in;
         for (int i = 0; i < nb * nb; ++i)
-            if (h->launches_direct[i].pp <= kMmaDegree && mma_class(h->launches_direct[i].pp) == cls) in.push_back(i);
+            if (h->launches_direct[i].pp <= kMmaDegree && mma_class(h->launches_direct[i].pp, sum) == cls) in.push_back(i);
         if (in.empty()) continue;
         std::stable_sort(in.begin(), in.end(),
                          [&](int a, int b) { return h->launches_direct[a].pp > h->launches_direct[b].pp; });
         const int pp = h->launches_direct[in[0]].pp;
-        const int slots = 148 * mma_ctas_per_sm(pp);
+        const int slots = 148 * mma_ctas_per_sm(pp, sum);
         auto chunks_for = [&](int i, int B) {
             const int batches = (h->launches_direct[i].nsources + 3) / 4;
             return std::max(1, std::min({per, batches, (batches + B - 1) / B}));
@@ -667,7 +669,7 @@ int make_mma_plan(foggy_handle h, int nrhs, MmaPlan& p) {
     int id = 0;
     for (int q = 0; q < 12; ++q) {
         p.use.of[q] = (unsigned char)id;
-        id += std::any_of(h->p_s.begin(), h->p_s.end(), [&](int pj) { return (pj - 1) / 4 == q; });
+        id += std::any_of(h->p_s.begin(), h->p_s.end(), [&](int pj) { return pj / 4 == q; });
     }
     if (work.empty()) return FOGGY_OK;
     TRY(dalloc(h, &p.d_work, work.size()));
@@ -675,12 +677,13 @@ int make_mma_plan(foggy_handle h, int nrhs, MmaPlan& p) {
     return FOGGY_OK;
 }
 
-int mma_plan(foggy_handle h, int nrhs, const MmaPlan** out) {
-    auto it = h->mma_plans.find(nrhs);
+int mma_plan(foggy_handle h, int nrhs, bool sum, const MmaPlan** out) {
+    const auto key = std::make_pair(nrhs, sum);
+    auto it = h->mma_plans.find(key);
     if (it == h->mma_plans.end()) {
         MmaPlan p;
-        TRY(make_mma_plan(h, nrhs, p));
-        it = h->mma_plans.emplace(nrhs, std::move(p)).first;
+        TRY(make_mma_plan(h, nrhs, sum, p));
+        it = h->mma_plans.emplace(key, std::move(p)).first;
     }
     *out = &it->second;
     return FOGGY_OK;
@@ -1444,7 +1447,7 @@ int apply_operator_fmm(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false
 // holds the plan's slabs
 int launch_mma(foggy_handle h, DirectArgs a, int nrhs, const cplx* X, cplx* Y) {
     const MmaPlan* p = nullptr;
-    TRY(mma_plan(h, nrhs, &p));
+    TRY(mma_plan(h, nrhs, a.pt.stab == nullptr, &p));
     const MmaTabs mt = mma_tabs(h);
     const int nv = std::max(1, nrhs);
     a.x = X;
@@ -1548,7 +1551,7 @@ void free_scene(foggy_handle h) {
     dfree(h, h->d_partial);
     dfree(h, h->d_bslab);
     h->bslab_vectors = 0;
-    for (auto& [nrhs, p] : h->mma_plans) dfree(h, p.d_work);
+    for (auto& [key, p] : h->mma_plans) dfree(h, p.d_work);
     h->mma_plans.clear();
     dfree(h, h->d_stab);
     dfree(h, h->d_stab32);

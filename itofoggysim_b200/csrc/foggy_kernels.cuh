@@ -144,10 +144,10 @@ struct MmaTabs {
 };
 void build_mma_tables(int pmax, const std::vector<double>& delta, std::vector<double>& frag, std::vector<double>& wf,
                       std::vector<int>& plan);
-// CTAs of a launch of largest degree pp that an SM holds at once
-int mma_ctas_per_sm(int pp);
-// the kernel instantiation of a largest degree, 0..3: launches of one class go as one
-int mma_class(int pp);
+// CTAs of a launch of largest degree pp that an SM holds at once (sum: without pair tables)
+int mma_ctas_per_sm(int pp, bool sum);
+// the kernel instantiation of a largest degree, 0..4: launches of one class go as one
+int mma_class(int pp, bool sum);
 // A (target bucket, source bucket) share of a launch: CTAs cta0 .. cta0 + ntargets nrhs chunks - 1, vector fastest, then
 // target, then chunk
 struct MmaWork {
@@ -207,7 +207,7 @@ struct PairArgs {
 size_t pair_s_group_smem_bytes(int M2);
 void launch_pair_s_group(const PairArgs& a, int tile0, int ntiles, int M2, cudaStream_t s);
 // Which slabs a final sum reads: per right-hand side `per_rhs` slabs, source bucket s's from s per_bucket on; the
-// target's bucket of[(p - 1) / 4] fills c[bucket][s] of them.  nb = 0: the first per_rhs slabs, whatever the sphere.
+// target's bucket of[p / 4] fills c[bucket][s] of them.  nb = 0: the first per_rhs slabs, whatever the sphere.
 struct SlabUse {
     int nb, per_rhs, per_bucket;
     unsigned char of[12];

@@ -1486,7 +1486,7 @@ __global__ void k_direct_finish(SceneView sc, const cplx* x, const cplx* partial
     x += blockIdx.y * ld;
     y += blockIdx.y * ld;
     partial += (size_t)blockIdx.y * use.per_rhs * n_unk;
-    const int row = use.nb ? use.of[(pj - 1) >> 2] : 0;
+    const int row = use.nb ? use.of[pj >> 2] : 0;
     for (int t = threadIdx.x; t < 2 * Pj; t += blockDim.x) {
         cplx v = x[o + t];
         if (cp) {

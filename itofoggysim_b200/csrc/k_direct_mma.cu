@@ -79,7 +79,7 @@ __device__ __forceinline__ void run_batches(const Shared& s, const MmaTabs& mt, 
         }
     };
 
-    for (int t = tid; t < kPlanInts; t += T) s.blk[t] = mt.plan[kPlanInts * pp + t];
+    for (int t = tid; t < kPlanInts; t += T) s.blk[t] = mt.plan[kPlanInts * (pp + (SUM ? kMmaDegree + 1 : 0)) + t];
     if (tid < 4) s.zero[tid] = make_double2(0.0, 0.0);
     for (int t = tid; t < 2 * Pj; t += T) s.acc[t] = make_double2(0.0, 0.0);
     for (int t = tid; t < 8 * NI + 8; t += T) s.rn[t] = t ? 0.5 / (double)(t * (t + 1)) : 0.0;
@@ -206,29 +206,27 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_translate_mma(TransArgs a, Mma
     }
 }
 
-int mma_ctas_per_sm(int pp) { return pp <= 7 ? 4 : pp <= 23 ? 2 : 1; }
-int mma_class(int pp) { return pp <= 7 ? 0 : pp <= 15 ? 1 : pp <= 23 ? 2 : 3; }
+int mma_ctas_per_sm(int pp, bool sum) { return pp <= 7 ? 4 : pp <= 19 ? 2 : pp <= 23 && !sum ? 2 : 1; }
+int mma_class(int pp, bool sum) { return pp <= 7 ? 0 : pp <= 15 ? 1 : pp <= 19 && sum ? 2 : pp <= 23 ? 3 : 4; }
 int mma_unit_size(int pp) { return mma::unit_size(pp); }
 
-// f(kernel tag) with the instantiation of a launch of largest degree pp
-template <class F>
+// f<NI, W, CTAS> of a launch of largest degree pp
+template <bool SUM, class F>
 static void by_degree(int pp, F f) {
-    if (pp <= 7) f.template operator()<1, mma::warps_of(7), 4>();
-    else if (pp <= 15) f.template operator()<2, mma::warps_of(15), 2>();
-    else if (pp <= 23) f.template operator()<3, mma::warps_of(23), 2>();
-    else f.template operator()<4, mma::warps_of(31), 1>();
+    if (pp <= 7) f.template operator()<1, mma::warps_of(7, SUM), 4>();
+    else if (pp <= 15) f.template operator()<2, mma::warps_of(15, SUM), 2>();
+    else if (pp <= 19) f.template operator()<3, mma::warps_of(19, SUM), 2>();
+    else if (pp <= 23) f.template operator()<3, mma::warps_of(23, SUM), SUM ? 1 : 2>();
+    else f.template operator()<4, mma::warps_of(31, SUM), 1>();
 }
 
 void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const MmaWork* w, int nw, int ctas, int pp, int nrhs,
                        int64_t ld, int per_rhs, bool after_other, cudaStream_t s) {
-    by_degree(pp, [&]<int NI, int W, int CTAS>() {
-        const bool sum = a.pt.stab == nullptr;
-        auto* kernel = sum ? k_direct_mma<NI, W, CTAS, true> : k_direct_mma<NI, W, CTAS, false>;
-        const size_t smem = mma::smem_bytes<NI>(pp) + (sum ? mma::sum_smem_bytes<NI>() : 0);
+    auto go = [&](auto* kernel, int warps, size_t smem) {
         raise_smem_ceiling(reinterpret_cast<const void*>(kernel), smem);
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)ctas);
-        cfg.blockDim = dim3(32 * W);
+        cfg.blockDim = dim3(32 * warps);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
         cudaLaunchAttribute at{};
@@ -237,11 +235,17 @@ void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const MmaWork* w,
         cfg.attrs = &at;
         cfg.numAttrs = after_other ? 1 : 0;
         cudaLaunchKernelEx(&cfg, kernel, a, mt, w, nw, nrhs, ld, per_rhs);
-    });
+    };
+    if (a.pt.stab)
+        by_degree<false>(pp, [&]<int NI, int W, int CTAS>() { go(k_direct_mma<NI, W, CTAS, false>, W, mma::smem_bytes<NI>(pp)); });
+    else
+        by_degree<true>(pp, [&]<int NI, int W, int CTAS>() {
+            go(k_direct_mma<NI, W, CTAS, true>, W, mma::smem_bytes<NI>(pp) + mma::sum_smem_bytes<NI>());
+        });
 }
 
 void launch_translate_mma(const TransArgs& a, const MmaTabs& mt, int pp, int ntargets, int chunks, cudaStream_t s) {
-    by_degree(pp, [&]<int NI, int W, int CTAS>() {
+    by_degree<false>(pp, [&]<int NI, int W, int CTAS>() {
         auto* kernel = k_translate_mma<NI, W, CTAS>;
         const size_t smem = mma::smem_bytes<NI>(pp);
         raise_smem_ceiling(reinterpret_cast<const void*>(kernel), smem);
@@ -269,8 +273,12 @@ void build_mma_tables(int pmax, const std::vector<double>& delta, std::vector<do
                                 frag.push_back(in <= n && out <= n ? Q[(size_t)in * (n + 1) + out] : 0.0);
                             }
     }
-    plan.assign((size_t)mma::kPlanInts * (kMmaDegree + 1), 0);
-    for (int pp = 1; pp <= kMmaDegree; ++pp) mma::make_plan(pp, mma::warps_of(pp), plan.data() + (size_t)mma::kPlanInts * pp);
+    // with tables, then without
+    plan.assign((size_t)2 * mma::kPlanInts * (kMmaDegree + 1), 0);
+    for (int sum = 0; sum < 2; ++sum)
+        for (int pp = 1; pp <= kMmaDegree; ++pp)
+            mma::make_plan(pp, mma::warps_of(pp, sum != 0),
+                           plan.data() + (size_t)mma::kPlanInts * (pp + sum * (kMmaDegree + 1)));
     // rows padded: the coaxial step reads whole k-steps of 4
     const int ld = pmax + 8;
     wf.assign(2 * (size_t)(pmax + 1) * ld, 0.0);

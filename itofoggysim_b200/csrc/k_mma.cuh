@@ -203,8 +203,9 @@ inline void make_plan(int pp, int warps, int* out) {
         o += frags_of(n);
     }
 }
-// warps of a launch's CTAs (launch_direct_mma)
-__host__ __device__ constexpr int warps_of(int pp) { return pp <= 7 ? 4 : pp <= 23 ? 8 : 12; }
+// warps of a launch's CTAs (by_degree); with S summed (sum) the radial functions leave no room for a second CTA on an
+// SM above order 19, so that one has twice the warps up to 23
+__host__ __device__ constexpr int warps_of(int pp, bool sum) { return pp <= 7 ? 4 : pp <= 19 ? 8 : pp <= 23 ? (sum ? 16 : 8) : 12; }
 
 // ---- rotation -----------------------------------------------------------------------------------------
 // Products of one degree's fragments with the folded input: for every output order i' = 8t + 4e + q
