@@ -509,7 +509,7 @@ DTabs dtabs(foggy_handle h) {
 }
 
 MmaTabs mma_tabs(foggy_handle h) {
-    return MmaTabs{reinterpret_cast<const double2*>(h->d_frag), reinterpret_cast<const double2*>(h->d_wf),
+    return MmaTabs{h->d_frag, reinterpret_cast<const double2*>(h->d_wf),
                    h->d_plan, h->tab_pmax + 8};
 }
 

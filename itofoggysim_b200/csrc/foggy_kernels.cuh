@@ -137,7 +137,7 @@ void launch_direct(const DirectArgs& a, const DirectBucket& b, cudaStream_t s);
 // k_direct_mma.cu -- the FP64 operator on the tensor cores, for orders up to kMmaDegree over the pair tables
 constexpr int kMmaDegree = 31;
 struct MmaTabs {
-    const double2* frag;       // d^n(pi/2) as fragments, degree by degree (build_mma_tables)
+    const double* frag;        // d^n(pi/2) as fragments, degree by degree (build_mma_tables)
     const double2* wf;         // factors of the coaxial step's w, one entry per (order, degree)
     const int* plan;           // shared-memory layouts and warps' degrees by largest degree
     int ld;                    // degrees per order of wf

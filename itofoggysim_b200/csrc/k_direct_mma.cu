@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_translate_mma(TransArgs a, Mma
     }
 }
 
-int mma_ctas_per_sm(int pp, bool sum) { return pp <= 7 ? 4 : pp <= 19 ? 2 : pp <= 23 && !sum ? 2 : 1; }
+int mma_ctas_per_sm(int pp, bool sum) { return pp <= 7 ? 4 : pp <= 15 ? (sum ? 2 : 3) : pp <= 19 ? 2 : pp <= 23 && !sum ? 2 : 1; }
 int mma_class(int pp, bool sum) { return pp <= 7 ? 0 : pp <= 15 ? 1 : pp <= 19 && sum ? 2 : pp <= 23 ? 3 : 4; }
 int mma_unit_size(int pp) { return mma::unit_size(pp); }
 
@@ -214,7 +214,7 @@ int mma_unit_size(int pp) { return mma::unit_size(pp); }
 template <bool SUM, class F>
 static void by_degree(int pp, F f) {
     if (pp <= 7) f.template operator()<1, mma::warps_of(7, SUM), 4>();
-    else if (pp <= 15) f.template operator()<2, mma::warps_of(15, SUM), 2>();
+    else if (pp <= 15) f.template operator()<2, mma::warps_of(15, SUM), SUM ? 2 : 3>();
     else if (pp <= 19) f.template operator()<3, mma::warps_of(19, SUM), 2>();
     else if (pp <= 23) f.template operator()<3, mma::warps_of(23, SUM), SUM ? 1 : 2>();
     else f.template operator()<4, mma::warps_of(31, SUM), 1>();
@@ -260,15 +260,15 @@ void build_mma_tables(int pmax, const std::vector<double>& delta, std::vector<do
     frag.clear();
     for (int n = 1; n <= pmax; ++n) {
         const double* Q = delta.data() + (size_t)n * (n + 1) * (2 * n + 1) / 6;
-        const int tiles = (mma::steps_of(n) + 1) / 2;
+        const int K = mma::steps_of(n);
         for (int P = 0; P < 2; ++P)
-            for (int t = 0; t < tiles; ++t)
+            for (int t = 0; t < (K + 1) / 2; ++t)
                 for (int r = 0; r < 2; ++r)
-                    for (int jp = 0; jp < tiles; ++jp)
+                    for (int j = 0; j < K; j += 2)
                         for (int lane = 0; lane < 32; ++lane)
-                            for (int e = 0; e < 2; ++e) {
+                            for (int e = 0; e < (j + 1 < K ? 2 : 1); ++e) {
                                 const int c = lane >> 2;   // column: output order 8t + 4 (c & 1) + c / 2
-                                const int in = 2 * (4 * (2 * jp + e) + (lane & 3)) + r;
+                                const int in = 2 * (4 * (j + e) + (lane & 3)) + r;
                                 const int out = 2 * (8 * t + 4 * (c & 1) + (c >> 1)) + P;
                                 frag.push_back(in <= n && out <= n ? Q[(size_t)in * (n + 1) + out] : 0.0);
                             }

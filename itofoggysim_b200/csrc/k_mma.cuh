@@ -58,11 +58,11 @@ __device__ __forceinline__ void mma8x8x4(double (&c)[2], double a, double b) {
 // ---- the Delta fragments --------------------------------------------------------------------------
 // degree n has n/2 + 1 even and (n+1)/2 odd orders >= 0: steps of 4 for either, output tiles of 8
 __host__ __device__ inline int steps_of(int n) { return (n / 2 + 4) / 4; }
-// fragments (32 lanes x double2, two k-steps each) of degree n: output parity, tile, input parity,
-// pair of k-steps
+// fragments of degree n, in doubles: output parity, tile, input parity, k-steps (32 lanes each; a pair's two values side
+// by side in a lane)
 __host__ __device__ inline int frags_of(int n) {
-    const int t = (steps_of(n) + 1) / 2;
-    return 4 * t * t;
+    const int k = steps_of(n);
+    return 4 * ((k + 1) / 2) * k * 32;
 }
 
 // ---- shared memory ----------------------------------------------------------------------------------
@@ -173,8 +173,9 @@ __device__ inline Shared carve(void* base, int pp, int us) {
 }
 
 // What a launch of largest degree pp lays out in shared memory, made on the host: the order offsets, the degrees
-// 1..pp dealt to the warps (largest first, each to the warp with the least work so far; one fragment of a degree is
-// one unit of work, and its loads and phases about four), each warp's first, and the first fragment of a degree.
+// 1..pp dealt to the warps (largest first, each to the warp with the least work so far), each warp's first, and the first
+// fragment of a degree.
+constexpr int kDegreeCost[4] = {10, 14, 26, 33};   // by k-steps: products, phases and load latencies, 100 cycles
 inline void make_plan(int pp, int warps, int* out) {
     int o = 0;
     for (int k = 0; k <= pp; ++k) {
@@ -187,7 +188,7 @@ inline void make_plan(int pp, int warps, int* out) {
         int b = 0;
         for (int w = 1; w < warps; ++w)
             if (load[w] < load[b]) b = w;
-        load[b] += frags_of(n) + 4;
+        load[b] += kDegreeCost[steps_of(n) - 1];
         own[n] = b;
     }
     o = 0;
@@ -212,7 +213,7 @@ __host__ __device__ constexpr int warps_of(int pp, bool sum) { return pp <= 7 ? 
 // of parity P, f(P, 2t + e, E, O) gets the sums over even and odd input orders.  A0 holds the input
 // for even output orders, A1 for odd ones, [input parity][k-step][re, im].
 template <int N, class F>
-__device__ __forceinline__ void delta_mul(const double2* __restrict__ frag, const double (&A0)[2][N][2],
+__device__ __forceinline__ void delta_mul(const double* __restrict__ frag, int lane, const double (&A0)[2][N][2],
                                           const double (&A1)[2][N][2], F f) {
     int at = 0;
 #pragma unroll
@@ -225,15 +226,16 @@ __device__ __forceinline__ void delta_mul(const double2* __restrict__ frag, cons
                 acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.0;
 #pragma unroll
                 for (int j = 0; j < N; j += 2) {
-                    const double2 b = __ldg(frag + 32 * at);
-                    ++at;
                     const double a0 = P ? A1[r][j][0] : A0[r][j][0], a1 = P ? A1[r][j][1] : A0[r][j][1];
                     if (j + 1 < N) {
                         const double a2 = P ? A1[r][j + 1][0] : A0[r][j + 1][0];
                         const double a3 = P ? A1[r][j + 1][1] : A0[r][j + 1][1];
+                        const double2 b = __ldg(reinterpret_cast<const double2*>(frag + 32 * at) + lane);
                         mma16x8x8(acc[r], a0, a1, a2, a3, b.x, b.y);
+                        at += 2;
                     } else {
-                        mma16x8x4(acc[r], a0, a1, b.x);
+                        mma16x8x4(acc[r], a0, a1, __ldg(frag + 32 * at + lane));
+                        at += 1;
                     }
                 }
             }
@@ -276,7 +278,7 @@ struct Lane {
 // odd orders by unit bit 0, eight lanes away.  One function for both directions: the kernel's code has to
 // stay within the instruction cache.
 template <int NI, int N>
-__device__ __forceinline__ void rotate(const Shared& s, const Lane<NI>& L, const double2* __restrict__ frag, int n,
+__device__ __forceinline__ void rotate(const Shared& s, const Lane<NI>& L, const double* __restrict__ frag, int n,
                                        int pj, const Unit& un, int cur, bool out) {
     const int q = L.q;
     const double2* eps = s.eps + (cur * kUnits + L.u) * phase_ld<NI>() + 2 * q;
@@ -332,7 +334,7 @@ __device__ __forceinline__ void rotate(const Shared& s, const Lane<NI>& L, const
     // folded input of the second product from the sums of the first:
     //   even outputs (-1)^s (2 cos E - 2i sin O), odd ones (-1)^s (2 cos O - 2i sin E)
     double B0[2][N][2], B1[2][N][2];
-    delta_mul<N>(frag, A0, A1, [&](int P, int j, cplx E, cplx O) {
+    delta_mul<N>(frag, L.lane, A0, A1, [&](int P, int j, cplx E, cplx O) {
         const double2 h = eth[2 * (4 * j + q) + P];
         B0[P][j][0] = fma(h.y, O.y, h.x * E.x);
         B0[P][j][1] = fma(-h.y, O.x, h.x * E.y);
@@ -340,7 +342,7 @@ __device__ __forceinline__ void rotate(const Shared& s, const Lane<NI>& L, const
         B1[P][j][1] = fma(-h.y, E.x, h.x * O.y);
     });
     // sums of the second product, over the first's input
-    delta_mul<N>(frag, B0, B1, [&](int P, int j, cplx E, cplx O) {
+    delta_mul<N>(frag, L.lane, B0, B1, [&](int P, int j, cplx E, cplx O) {
         A0[P][j][0] = E.x;
         A0[P][j][1] = E.y;
         A1[P][j][0] = O.x;
@@ -394,13 +396,13 @@ __device__ __forceinline__ void rotate(const Shared& s, const Lane<NI>& L, const
 
 // degrees of one warp
 template <int NI>
-__device__ __forceinline__ void rotate_all(const Shared& s, const Lane<NI>& L, const double2* __restrict__ frag, int warp,
+__device__ __forceinline__ void rotate_all(const Shared& s, const Lane<NI>& L, const double* __restrict__ frag, int warp,
                                            int top, int pj, const Unit& un, int cur, bool out) {
 #pragma unroll 1
     for (int i = s.wfirst[warp]; i < s.wfirst[warp + 1]; ++i) {
         const int n = s.ord[i];
         if (n > top) continue;
-        const double2* f = frag + 32 * s.fo[n] + L.lane;
+        const double* f = frag + s.fo[n];
         switch (steps_of(n)) {
             case 1: rotate<NI, 1>(s, L, f, n, pj, un, cur, out); break;
             case 2: if constexpr (NI >= 2) rotate<NI, 2>(s, L, f, n, pj, un, cur, out); break;
@@ -429,17 +431,8 @@ __device__ __forceinline__ double2 ld_stream(const double2* p) {
     return v;
 }
 
-// S fragments of one tile of degrees n0 + r (clamped to pj: rows past it are not stored): k-steps mu = k + 4t + q,
-// clamped to pl + 1 in the last two steps (the next order may have a step less)
-template <int NT, int KT>
-__device__ __forceinline__ void load_s(double2 (&v)[KT], const Unit& un, int k, int n0, int pj, int lane) {
-    const int q = lane & 3;
-    const int M2 = (pj > un.p ? pj : un.p) + 2, Wk = M2 - k, top = un.p + 1 - k;
-    const double2* S = un.s + (block_offset(k, M2) + (min(n0 + (lane >> 2), pj) - k) * Wk);
-#pragma unroll
-    for (int t = 0; t < NT; ++t) v[t] = ld_stream(t >= NT - 2 ? S + min(4 * t + q, top) : S + q + 4 * t);
-}
-
+// S fragments of a tile of degrees n0 + r (clamped to pj: rows past it are not stored): k-steps mu = k + 4t + q, clamped
+// to pl + 1 in the last two steps (the next order may have a step less).
 // One order of one unit, tiles of eight degrees.  sv holds the first tile's fragments on entry and those of order
 // k + dk on exit.  One instantiation per number of k-steps NT = ceil((pl + 2 - k) / 4), so that the loops over
 // them carry no conditions.
@@ -486,14 +479,25 @@ __device__ __forceinline__ void coaxial_k(const Shared& s, const Unit& un, int u
     double2* Y = X + 4 * r + q;
 #pragma unroll 1
     for (int n0 = lo; n0 <= pj; n0 += 8, Y += 32) {
+        // the next tile's fragments, or the next order's first tile's, follow each product that frees theirs
+        const bool more = n0 + 8 <= pj, go = more || k + dk <= un.km;
+        const int kn = more ? k : k + dk, top = pl + 1 - kn;
+        const int M2 = (pj > pl ? pj : pl) + 2, Wk = M2 - kn;
+        const double2* S = un.s + (block_offset(kn, M2) + (min((more ? n0 + 8 : kn) + r, pj) - kn) * Wk);
+        auto reload = [&](int t) { sv[t] = ld_stream(t >= NT - 2 ? S + min(4 * t + q, top) : S + q + 4 * t); };
         double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-        for (int t = 0; t + 1 < NT; t += 2)
+        for (int t = 0; t + 1 < NT; t += 2) {
             mma16x8x8(acc, sv[t].x, sv[t].y, sv[t + 1].x, sv[t + 1].y, w[t], w[t + 1]);
-        if (NT & 1) mma16x8x4(acc, sv[NT - 1].x, sv[NT - 1].y, w[NT - 1]);
-        // the next tile, or the next order's first
-        const bool more = n0 + 8 <= pj;
-        if (more || k + dk <= un.km) load_s<NT>(sv, un, more ? k : k + dk, more ? n0 + 8 : k + dk, pj, lane);
+            if (go) {
+                reload(t);
+                reload(t + 1);
+            }
+        }
+        if (NT & 1) {
+            mma16x8x4(acc, sv[NT - 1].x, sv[NT - 1].y, w[NT - 1]);
+            if (go) reload(NT - 1);
+        }
         const int n = n0 + r;
         const double g = flip(s.rn[n], fm);
         if (n <= pj) Y[0] = make_double2(g * (acc[0] - acc[3]), g * (acc[1] + acc[2]));
