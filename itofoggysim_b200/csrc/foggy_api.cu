@@ -955,7 +955,8 @@ void free_fmm(foggy_handle h) {
 // few boxes still fill the GPU; their partial sums need fewer than 2 kFmmFill slabs of one target.
 constexpr int kFmmFill = 148 * 6;
 constexpr int kFmmChunks = 16;
-// list entries from which a pass runs on the tensor cores
+// list entries from which a pass runs on the tensor cores: below, its time is a launch or two either way.  500 long-wave
+// spheres, per application: near field 318 -> 93 us; M2L (levels of orders 17 and 11) 855 -> 350 us.
 constexpr int kFmmMmaEntries = 4096;
 
 // Expansion order of the boxes of level l.  The reference expands every box to its global order
@@ -1405,31 +1406,29 @@ int apply_operator_fmm(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false
         h->launches += chunks > 1 ? 2 : 1;
     };
     // On the tensor cores: cached blocks, orders up to kMmaDegree, lists of four sources and more (a shorter list
-    // leaves units of its batch empty) and enough of them that the pass is not its launch's latency alone.
-    auto takes_mma = [&](const FmmPass& q, int pp) {
+    // leaves units of its batch empty), in a pass of kFmmMmaEntries entries and more.
+    auto takes_mma = [&](const FmmPass& q, int pp, int pass_entries) {
         int longest = 0;
-        const int entries = list_of(q, longest);
-        return h->d_fmm_taboff && pp <= kMmaDegree && entries >= 4 * q.ntgt && entries >= kFmmMmaEntries;
+        return h->d_fmm_taboff && pp <= kMmaDegree && list_of(q, longest) >= 4 * q.ntgt && pass_entries >= kFmmMmaEntries;
     };
     for (size_t i = 0; i < passes.size(); ++i) {
         const FmmPass& q = passes[i];
         Trace tp(names[stage[i]]);
-        if (stage[i] == 2) {
-            // M2L: one launch, unless its size pays for one per level with that level's order
-            int longest = 0;
-            if (h->d_fmm_taboff && list_of(q, longest) >= kFmmMmaEntries) {
-                for (int li = 0; li < nlev; ++li) {
-                    FmmPass ql = q;
-                    ql.tbase = t.level_base[li];
-                    ql.ntgt = t.level_base[li + 1] - ql.tbase;
-                    const int pp = h->fmm_order[li];
-                    launch(ql, false, takes_mma(ql, pp) ? pp : 0);
-                }
-                continue;
+        int longest = 0;
+        const int entries = list_of(q, longest);
+        if (stage[i] == 2 && h->d_fmm_taboff && entries >= kFmmMmaEntries) {
+            // M2L of this size: one launch per level with that level's order
+            for (int li = 0; li < nlev; ++li) {
+                FmmPass ql = q;
+                ql.tbase = t.level_base[li];
+                ql.ntgt = t.level_base[li + 1] - ql.tbase;
+                const int pp = h->fmm_order[li];
+                launch(ql, false, takes_mma(ql, pp, entries) ? pp : 0);
             }
+            continue;
         }
-        const int pp = stage[i] == 5 ? std::max(h->pmax, 1) : base.pp;
-        launch(q, stage[i] == 5, (stage[i] == 5 && takes_mma(q, pp)) ? pp : 0);
+        const int pp = std::max(h->pmax, 1);
+        launch(q, stage[i] == 5, (stage[i] == 5 && takes_mma(q, pp, entries)) ? pp : 0);
     }
     // join first, so that whatever follows on the handle's stream (frees included) comes after the side
     cudaEventRecord(h->ev_join, h->side);
