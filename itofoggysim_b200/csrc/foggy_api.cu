@@ -1443,8 +1443,8 @@ int apply_operator_fmm(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false
 }
 
 // Y_r = A X_r on the tensor cores for the nrhs vectors X + r n_unk (nrhs = 0: foggy_matvec_static's one); a.partial
-// holds the plan's slabs
-int launch_mma(foggy_handle h, DirectArgs a, int nrhs, const cplx* X, cplx* Y) {
+// holds the plan's slabs.  xref given: one vector, Y and xref in the reference layout.
+int launch_mma(foggy_handle h, DirectArgs a, int nrhs, const cplx* X, cplx* Y, const cplx* xref = nullptr) {
     const MmaPlan* p = nullptr;
     TRY(mma_plan(h, nrhs, a.pt.stab == nullptr, &p));
     const MmaTabs mt = mma_tabs(h);
@@ -1453,7 +1453,10 @@ int launch_mma(foggy_handle h, DirectArgs a, int nrhs, const cplx* X, cplx* Y) {
     for (const MmaPlan::Launch& l : p->launches)
         launch_direct_mma(a, mt, p->d_work + l.first, l.count, l.ctas, l.pp, nv, h->n_unk, p->use.per_rhs,
                           &l != &p->launches.front(), h->stream);
-    k_direct_finish<<<dim3(h->N, nv), 256, 0, h->stream>>>(a.sc, X, a.partial, p->use, h->n_unk, h->n_unk, Y);
+    if (xref)
+        k_direct_finish_pack<<<h->N, 256, 0, h->stream>>>(a.sc, X, a.partial, p->use, h->n_unk, h->pg, h->d_g, xref, Y);
+    else
+        k_direct_finish<<<dim3(h->N, nv), 256, 0, h->stream>>>(a.sc, X, a.partial, p->use, h->n_unk, h->n_unk, Y);
     h->launches += (int64_t)p->launches.size() + 1;
     CKL(h);
     return FOGGY_OK;
@@ -2164,8 +2167,18 @@ int32_t foggy_matvec(foggy_handle h, const double* x, double* y, int32_t mem) {
     }
     SceneView sv = scene_view(h);
     k_unpack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, xr, h->d_tmp_in);
-    TRY(apply_operator(h, h->d_tmp_in, h->d_tmp_out));
-    k_pack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, h->d_tmp_out, xr, yr);
+    bool packed = false;
+    if (h->prm.matvec_mode == FOGGY_MATVEC_DIRECT) {
+        TRY(ensure_pair_tables(h));
+        const DirectArgs a = direct_args(h, h->d_tmp_in);
+        packed = mma_operator(h, a);
+        Trace tr("operator (FP64)");
+        if (packed) TRY(launch_mma(h, a, 1, h->d_tmp_in, yr, xr));
+    }
+    if (!packed) {
+        TRY(apply_operator(h, h->d_tmp_in, h->d_tmp_out));
+        k_pack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, h->d_tmp_out, xr, yr);
+    }
     CKL(h);
     if (mem == FOGGY_MEM_HOST)
         CK(h, cudaMemcpyAsync(y, yr, len * sizeof(cplx), cudaMemcpyDeviceToHost, h->stream));

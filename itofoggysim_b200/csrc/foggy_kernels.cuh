@@ -217,6 +217,9 @@ struct SlabUse {
 // ld entries apart)
 __global__ void k_direct_finish(SceneView sc, const cplx* x, const cplx* partial, SlabUse use, int64_t n_unk, int64_t ld,
                                 cplx* y);
+// the same of one vector into the reference layout, identity rows from xref
+__global__ void k_direct_finish_pack(SceneView sc, const cplx* x, const cplx* partial, SlabUse use, int64_t n_unk, int pg,
+                                     const double* g, const cplx* xref, cplx* yref);
 // Sphere or box centres with their truncation orders and the offsets of their coefficient
 // vectors (scaled basis, a then b, standard (n, m) order).
 struct PointSet {

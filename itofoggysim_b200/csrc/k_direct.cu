@@ -1475,43 +1475,60 @@ bool launch_direct_block(const BlockArgs& a, const DirectBucket& b, int R, cudaS
     return false;
 }
 
+// x + T (sum of the slabs) of entry t of sphere j (t over the a part, then the b part); see SlabUse
+__device__ __forceinline__ cplx finished(const SceneView& sc, const cplx* x, const cplx* partial, const SlabUse& use,
+                                         int64_t n_unk, int j, int pj, int t) {
+    const int Pj = pj * (pj + 2);
+    const int64_t o = sc.off[j] + t;
+    const cplx v = x[o];
+    if (!sc.couple[j]) return v;
+    const int row = use.nb ? use.of[pj >> 2] : 0;
+    cplx sum = mk(0, 0);
+    for (int b = 0; b < (use.nb ? use.nb : 1); ++b) {
+        const cplx* q = partial + (size_t)b * use.per_bucket * n_unk + o;
+        const int m = use.nb ? use.c[row][b] : use.per_rhs;
+        int c = 0;
+        for (; c + 4 <= m; c += 4) {   // four loads in flight, added in order
+            const cplx q0 = q[(size_t)c * n_unk], q1 = q[(size_t)(c + 1) * n_unk], q2 = q[(size_t)(c + 2) * n_unk],
+                       q3 = q[(size_t)(c + 3) * n_unk];
+            sum = sum + q0;
+            sum = sum + q1;
+            sum = sum + q2;
+            sum = sum + q3;
+        }
+        for (; c < m; ++c) sum = sum + q[(size_t)c * n_unk];
+    }
+    int n, m;
+    decode_nm(t < Pj ? t : t - Pj, n, m);
+    const cplx tm = (t < Pj) ? sc.an[(size_t)j * sc.pmax + n - 1] : sc.bn[(size_t)j * sc.pmax + n - 1];
+    return v + tm * sum;
+}
+
 // y = x + T (sum of the slabs) for coupled spheres, y = x otherwise
 __global__ void k_direct_finish(SceneView sc, const cplx* x, const cplx* partial, SlabUse use, int64_t n_unk, int64_t ld,
                                 cplx* y) {
-    int j = blockIdx.x;
-    int pj = sc.p[j];
-    int Pj = pj * (pj + 2);
-    int64_t o = sc.off[j];
-    bool cp = sc.couple[j] != 0;
+    const int j = blockIdx.x, pj = sc.p[j];
     x += blockIdx.y * ld;
     y += blockIdx.y * ld;
     partial += (size_t)blockIdx.y * use.per_rhs * n_unk;
-    const int row = use.nb ? use.of[pj >> 2] : 0;
-    for (int t = threadIdx.x; t < 2 * Pj; t += blockDim.x) {
-        cplx v = x[o + t];
-        if (cp) {
-            cplx sum = mk(0, 0);
-            for (int b = 0; b < (use.nb ? use.nb : 1); ++b) {
-                const cplx* q = partial + (size_t)b * use.per_bucket * n_unk + o + t;
-                const int m = use.nb ? use.c[row][b] : use.per_rhs;
-                int c = 0;
-                for (; c + 4 <= m; c += 4) {   // four loads in flight, added in order
-                    const cplx q0 = q[(size_t)c * n_unk], q1 = q[(size_t)(c + 1) * n_unk],
-                               q2 = q[(size_t)(c + 2) * n_unk], q3 = q[(size_t)(c + 3) * n_unk];
-                    sum = sum + q0;
-                    sum = sum + q1;
-                    sum = sum + q2;
-                    sum = sum + q3;
-                }
-                for (; c < m; ++c) sum = sum + q[(size_t)c * n_unk];
-            }
-            int tt = t < Pj ? t : t - Pj;
+    for (int t = threadIdx.x; t < 2 * pj * (pj + 2); t += blockDim.x)
+        y[sc.off[j] + t] = finished(sc, x, partial, use, n_unk, j, pj, t);
+}
+
+// The same straight into the reference layout (k_pack with identity rows): one launch less in a single application
+__global__ void k_direct_finish_pack(SceneView sc, const cplx* x, const cplx* partial, SlabUse use, int64_t n_unk, int pg,
+                                     const double* g, const cplx* xref, cplx* yref) {
+    const int j = blockIdx.x, pj = sc.p[j], Pj = pj * (pj + 2), C = (pg + 1) * (pg + 1) - 1;
+    for (int e = threadIdx.x; e < 2 * C; e += blockDim.x) {
+        const int part = e >= C, t = e - part * C;
+        const size_t o = (size_t)2 * C * j + e;
+        if (t < Pj) {
             int n, m;
-            decode_nm(tt, n, m);
-            cplx tm = (t < Pj) ? sc.an[(size_t)j * sc.pmax + n - 1] : sc.bn[(size_t)j * sc.pmax + n - 1];
-            v = v + tm * sum;
+            decode_nm(t, n, m);
+            yref[o] = g[n * (n + 1) + m] * finished(sc, x, partial, use, n_unk, j, pj, part * Pj + t);
+        } else {
+            yref[o] = xref[o];   // above the sphere's own order
         }
-        y[o + t] = v;
     }
 }
 
