@@ -2836,6 +2836,7 @@ namespace {
 
 // Tile width R per launch shape, chosen by timing: (FP32, pair tables, largest degree, log2 of the
 // target count, block width up to 8) -> R.  Process-wide, as the choice depends on the shape only.
+constexpr size_t kBlockKeepBytes = (size_t)256 << 20;   // host vectors of foggy_matvec_block kept on the device
 constexpr size_t kBlockSlabBytes = (size_t)128 << 20;   // slabs of many vectors at once on the tensor cores
 std::mutex g_tile_mu;
 std::map<std::tuple<int, int, int, int, int>, int> g_tile_cache;
@@ -3230,34 +3231,52 @@ int32_t foggy_matvec_block(foggy_handle h, int32_t nrhs, int32_t precision, cons
         dfree(h, X);
         return rc;
     };
+    // the identity rows above a sphere's degree come from x: vectors from the host are kept while the pool gives room,
+    // else copied again
+    cplx* kept = nullptr;
+    if (mem == FOGGY_MEM_HOST && (size_t)nrhs * len * sizeof(cplx) <= kBlockKeepBytes &&
+        talloc(h, &kept, (size_t)nrhs * len * sizeof(cplx)) != cudaSuccess) {
+        cudaGetLastError();
+        kept = nullptr;
+    }
+    auto fin_x = [&](int rc) {
+        tfree(h, kept);
+        return fin(rc);
+    };
     for (int r = 0; r < nrhs; ++r) {
         const cplx* src = reinterpret_cast<const cplx*>(x) + r * len;
         if (mem == FOGGY_MEM_HOST) {
-            if (cudaMemcpyAsync(h->d_ref_a, src, len * sizeof(cplx), cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
-                return fin(fail(h, FOGGY_ERR_CUDA, "foggy_matvec_block: host to device copy"));
-            src = h->d_ref_a;
+            cplx* dst = kept ? kept + r * len : h->d_ref_a;
+            if (cudaMemcpyAsync(dst, src, len * sizeof(cplx), cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
+                return fin_x(fail(h, FOGGY_ERR_CUDA, "foggy_matvec_block: host to device copy"));
+            src = dst;
         }
         k_unpack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, src, X + (size_t)r * n);
     }
     int rc = apply_operator_block(h, X, Y, nrhs, precision == 1, precision == 1);
-    if (rc) return fin(rc);
+    if (rc) return fin_x(rc);
     for (int r = 0; r < nrhs; ++r) {
         const cplx* xr = reinterpret_cast<const cplx*>(x) + r * len;
         cplx* dst = reinterpret_cast<cplx*>(y) + r * len;
         if (mem == FOGGY_MEM_HOST) {
-            // the identity rows above a sphere's degree come from x, staged again
-            cudaMemcpyAsync(h->d_ref_a, xr, len * sizeof(cplx), cudaMemcpyHostToDevice, h->stream);
-            xr = h->d_ref_a;
-            k_pack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, Y + (size_t)r * n, xr, h->d_ref_b);
-            cudaMemcpyAsync(dst, h->d_ref_b, len * sizeof(cplx), cudaMemcpyDeviceToHost, h->stream);
+            cplx* out = h->d_ref_b;
+            if (kept) {
+                xr = out = kept + r * len;   // in place: each entry is read by the thread that writes it
+            } else {
+                cudaMemcpyAsync(h->d_ref_a, xr, len * sizeof(cplx), cudaMemcpyHostToDevice, h->stream);
+                xr = h->d_ref_a;
+            }
+            k_pack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, Y + (size_t)r * n, xr, out);
+            if (!kept) cudaMemcpyAsync(dst, out, len * sizeof(cplx), cudaMemcpyDeviceToHost, h->stream);
         } else {
             k_pack<<<h->N, 128, 0, h->stream>>>(sv, h->pg, h->d_g, Y + (size_t)r * n, xr, dst);
         }
     }
+    if (kept) cudaMemcpyAsync(y, kept, (size_t)nrhs * len * sizeof(cplx), cudaMemcpyDeviceToHost, h->stream);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return fin(fail(h, FOGGY_ERR_CUDA, std::string("foggy_matvec_block: ") + cudaGetErrorString(e)));
-    return fin(FOGGY_OK);
+    if (e != cudaSuccess) return fin_x(fail(h, FOGGY_ERR_CUDA, std::string("foggy_matvec_block: ") + cudaGetErrorString(e)));
+    return fin_x(FOGGY_OK);
 }
 
 int32_t foggy_solve_block(foggy_handle h, int32_t nrhs, const double* x0, double* x, int32_t mem, foggy_stats* stats,
