@@ -513,9 +513,9 @@ MmaTabs mma_tabs(foggy_handle h) {
                    h->d_plan, h->tab_pmax + 8};
 }
 
-// Whether the FP64 operator runs on the tensor cores: over the pair tables, orders up to kMmaDegree.  It is the
-// faster one at every order it takes (222 spheres of one order: 7 0.29 against 1.39 ms, 15 0.76 / 2.0, 23 1.83 / 4.9,
-// 31 3.7 / 9.7); without tables k_direct's seven stages sum S where they use it.
+// Whether the FP64 operator runs on the tensor cores: orders up to kMmaDegree, with the pair tables or without.  It is
+// the faster one at every order it takes (222 spheres of one order over tables: 7 0.29 against 1.39 ms, 15 0.75 / 2.0,
+// 23 1.8 / 4.9, 31 3.4 / 9.7; 211 spheres of orders 5..9 that sum S: 3.8 / 6.5).
 bool mma_operator(foggy_handle h, const DirectArgs&) { return h->pmax <= kMmaDegree; }
 
 DirectArgs direct_args(foggy_handle h, const cplx* x) {
@@ -813,9 +813,9 @@ int build_pair_tables(foggy_handle h, const SGaunt& g, bool fp64, bool fp32) {
 // cores, the single-precision ones tensor-core products in 3xTF32 (build_pair_tables).
 // A mixed-precision handle's Arnoldi steps run the FP64 tensor-core operator where its orders and tables allow: it is as
 // fast as the FP32 one, and its solve needs no refinement cycles (250 lognormal spheres to 1e-11: 260 ms with FP32
-// steps, 148 with these; 32 right-hand sides of 64 spheres: 160 and 114).  So such a handle keeps the double-precision tables
-// alone where they fit, and the single-precision ones where they do not, above kMmaDegree, or where FP32 is asked for
-// by name (fp32).
+// steps, 100 with these; 32 right-hand sides of 64 spheres: 159 and 101).  So such a handle keeps the double-precision
+// tables alone where they fit, and the single-precision ones where they do not, above kMmaDegree, or where FP32 is asked
+// for by name (fp32).
 int ensure_pair_tables(foggy_handle h, bool fp32 = false) {
     const bool mixed = h->prm.precision == 1;
     if (h->prm.pair_tables < 0 || h->N < 2) {
@@ -1749,7 +1749,7 @@ int gmres(foggy_handle h, foggy_stats* st) {
             status = FOGGY_OK;   // solve with the columns built so far
         }
         if (k > 0) {
-            k_trisolve<<<1, 1, 0, h->stream>>>(h->d_H, m, h->d_gv, k, h->d_y);
+            k_trisolve<<<1, 32, 0, h->stream>>>(h->d_H, m, h->d_gv, k, h->d_y);
             k_update_x<<<G, 256, 0, h->stream>>>(h->d_x, h->d_V, n, h->d_y, k, n);
             h->launches += 2;
         }
@@ -3191,7 +3191,7 @@ int block_gmres(foggy_handle h, int nrhs, foggy_stats* st, std::vector<int>& ite
             }
             if (!any || k + 1 >= steps) break;
         }
-        k_trisolve_b<<<(nact + 63) / 64, 64, 0, h->stream>>>(p.H, m, p.g, p.kend, p.y, nact);
+        k_trisolve_b<<<nact, 32, 0, h->stream>>>(p.H, m, p.g, p.kend, p.y);
         k_update_x_b<<<dim3(G, nact), 256, 0, h->stream>>>(h->d_bX, n, h->d_bV, ldi, p.y, m + 1, p.kend, n);
         h->launches += 2;
         CKL(h);

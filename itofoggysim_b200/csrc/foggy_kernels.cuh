@@ -292,7 +292,7 @@ __global__ void k_norm_partial(const cplx* w, int64_t n, double* part);
 __global__ void k_norm_reduce(const double* part, double* out);
 __global__ void k_scale_copy(const cplx* w, const double* nrm, cplx* v, int64_t n);
 __global__ void k_sub(const cplx* b, const cplx* ax, cplx* r, int64_t n);
-__global__ void k_trisolve(const cplx* H, int ldh, const cplx* g, int k, cplx* y);
+__global__ void __launch_bounds__(32) k_trisolve(const cplx* H, int ldh, const cplx* g, int k, cplx* y);
 __global__ void k_update_x(cplx* x, const cplx* V, int64_t ld, const cplx* y, int k, int64_t n);
 __global__ void k_init_cycle(cplx* g, int m1, const double* beta, int* flags);
 // several right-hand sides: one Krylov space per slot (blockIdx.y), basis vector i of slot b at
@@ -303,7 +303,7 @@ __global__ void k_scale_copy_b(const cplx* W, int64_t ldw, const double* nrm, in
                                int64_t n, const int* live);
 __global__ void k_sub_b(const cplx* Bv, const cplx* AX, cplx* Rv, int64_t ld, int64_t n);
 __global__ void k_init_cycle_b(cplx* g, int m1, const double* beta, int nslots, int* live, int* kend);
-__global__ void k_trisolve_b(const cplx* H, int m, const cplx* g, const int* kend, cplx* y, int nslots);
+__global__ void __launch_bounds__(32) k_trisolve_b(const cplx* H, int m, const cplx* g, const int* kend, cplx* y);
 __global__ void k_update_x_b(cplx* X, int64_t ld, const cplx* V, int64_t ldi, const cplx* y, int ystride,
                              const int* kend, int64_t n);
 
