@@ -1468,7 +1468,9 @@ int apply_operator(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false) {
     if (h->prm.matvec_mode == FOGGY_MATVEC_MLFMM) return apply_operator_fmm(h, x, y, fp32);
     TRY(ensure_pair_tables(h));
     DirectArgs a = direct_args(h, x);
-    const bool mma = mma_operator(h, a);   // also for the Arnoldi steps of a mixed-precision solve
+    // also for the Arnoldi steps of a mixed-precision solve, unless the single-precision tables alone fit: reading those
+    // beats summing S in FP64
+    const bool mma = mma_operator(h, a) && !(fp32 && h->stab32_ready && !h->stab_ready);
     a.fp32 = (!mma && fp32 && h->stab32_ready) ? 1 : 0;
     Trace tr(a.fp32 ? "operator (FP32)" : "operator (FP64)");
     if (mma) {
@@ -2944,7 +2946,7 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
     TRY(ensure_pair_tables(h, must32));
     const BlockArgs ba = block_args(h, X, Y, nrhs, fp32);
     // without tables the CUDA-core kernel sums S once for a tile of vectors
-    if (!must32 && mma_operator(h, ba.d) && (ba.d.pt.stab || nrhs == 1)) {
+    if (!must32 && mma_operator(h, ba.d) && (ba.d.pt.stab || (nrhs == 1 && !(fp32 && ba.d.pt.stab32)))) {
         // One vector per CTA: a batch's set-up that vectors could share is small beside its products, and the pair's
         // coaxial block comes from L2 after the first.  83 spheres, 5 right-hand sides to 1e-6: 161 -> 55 ms a request
         // (the tile autotuner's runs are gone too).  As many vectors at a time as have slabs: the handle's own, or a
@@ -2954,7 +2956,10 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
         DirectArgs a = ba.d;
         int most = h->cmax;
         const size_t one = (size_t)h->nbuckets * h->n_unk;
-        const int fit = (int)std::min<size_t>(nrhs, kBlockSlabBytes / (one * sizeof(cplx)));
+        // at most a quarter of what the budget leaves: a tight one is for the calls to come
+        const size_t room = (h->budget > h->bytes_in_use ? h->budget - h->bytes_in_use : 0) +
+                            (size_t)h->bslab_vectors * one * sizeof(cplx);
+        const int fit = (int)std::min<size_t>(nrhs, std::min(kBlockSlabBytes, room / 4) / (one * sizeof(cplx)));
         if (nrhs > most && fit > most) {
             if (h->bslab_vectors < fit) {
                 dfree(h, h->d_bslab);
