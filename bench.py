@@ -13,7 +13,7 @@ Printed JSON line (rank 0):
   value      solves/s of the whole job with the scene resident in HBM (device-timed, max over
              ranks), e2e the same through the public API with host buffers (scene upload,
              solve, solution download inside the timed region);
-  roofline   the operator kernel k_direct (>95% of the solve): achieved FP64 FLOP/s from the
+  roofline   the operator kernel k_direct_mma (>95% of the solve): achieved FP64 FLOP/s from the
              algorithmic flop count per launch and its CUDA-event time, against the FP64
              cuBLAS DGEMM rate measured in the same run;
   cpu_baseline  the FP64 oracle (restated reference algorithm, exact Xu translation
@@ -390,7 +390,7 @@ def run_serving(args):
         "metric": METRIC, "value": co["solves_s"], "unit": "solves/s", "n_gpus": 1, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": co["makespan_s"] * 1e3 / max(1, args.steps),
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f32 translations, f64 Krylov and residuals" if prec else "f64", "data": "synthetic",
+        "dtype": "f64 (up to order 31), f64 Krylov and residuals" if prec else "f64", "data": "synthetic",
         "config": {"workload": "serving stream: 50-500 lognormal spheres per request, 1-16 right-hand sides", "requests": args.steps,
                    "arrivals": "Poisson, 50 per s", "spheres": [int(min(r.n_spheres for r in timed)),
                                                                  int(max(r.n_spheres for r in timed))],
@@ -462,7 +462,8 @@ def block_scene(n_spheres):
 
 def run_block(args):
     """The 128 right-hand sides of one scene solved as one block in mixed precision
-    (foggy_solve_block: FP32 translation arithmetic in the Arnoldi steps, FP64 restart residuals,
+    (foggy_solve_block, precision 1: the FP64 tensor-core operator in the Arnoldi steps up to order 31 with tables,
+    FP32 translation arithmetic else; FP64 restart residuals,
     every operator application shared by the block), against the plain FP64 path (one FP64 GMRES per
     right-hand side, foggy_solve_rhs) on the same scene.  value = right-hand sides solved per second
     (device time of the block solve); errors of every right-hand side against the FP64 solutions."""
@@ -527,11 +528,12 @@ def run_block(args):
     line = {
         "metric": METRIC, "value": value, "unit": "rhs solves/s", "n_gpus": 1, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": float(np.mean(ms)), "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "f32 translations, f64 Krylov and residuals", "data": "synthetic",
+        "vs_baseline": None, "dtype": "f64 (up to order 31), f64 Krylov and residuals", "data": "synthetic",
         "config": {"workload": sc.name, "spheres": sc.n_spheres, "p_max": int(p.max()), "p_median": float(np.median(p)),
                    "rhs": nrhs, "gmres_restart": sc.gmres_restart, "gmres_tolerance": sc.gmres_tolerance,
                    "solver": "batched GMRES, one Krylov space per right-hand side, block operator",
-                   "matvec": "direct (all pairs, rotation-axial-rotation), right-hand-side tiles per CTA",
+                   "matvec": "direct (all pairs, rotation-axial-rotation); the roofline is of the FP32 block "
+                             "operator, asked for by name",
                    "l2": "Krylov block exceeds L2; 256 MB L2 flush between steps"},
         "plain_fp64": {"rhs_per_s": plain, "ms_total": st64["ms_total"], "iterations": st64["iterations"],
                        "solver": "foggy_solve_rhs: one FP64 GMRES per right-hand side"},
@@ -581,7 +583,7 @@ def run_operator(args):
         torch.cuda.synchronize()
         ms_first = (time.perf_counter() - t0) * 1e3   # wall time: pair tables, tile tuning, one application
         if args.solve:
-            # one GMRES(50) solve to 1e-8 instead (mixed precision: FP32 operator in the Arnoldi steps)
+            # one GMRES(50) solve to 1e-8 instead (mixed precision: see foggy_params.precision)
             s.set_restart(50)
             s.set_tolerance(1e-8)
             torch.cuda.profiler.start()
@@ -660,10 +662,11 @@ def g_layout(sc):
 
 
 def run_mixed(args):
-    """The workload solved with the FP32 operator in the Arnoldi steps and FP64 true residuals
+    """The workload solved by a mixed-precision handle (up to order 31 the FP64 tensor-core operator
+    serves the Arnoldi steps, above it the FP32 one) with FP64 true residuals
     (the 2000-sphere lognormal scene); value = solves/s (device time), with the relative error
     of the coefficients and of C_ext against one FP64 solve of the same scene.  The roofline is
-    that of the FP32 operator: its mean application time is the operator time of a solve less its
+    that of the Arnoldi steps' operator: its mean application time is the operator time of a solve less its
     FP64 residual applications (timed in the FP64 solve), over its Arnoldi steps."""
     import torch
     from itofoggysim_b200 import solver
@@ -702,29 +705,32 @@ def run_mixed(args):
            + sc.n_range_param.nbytes + 6 * 8 * sc.n_waves)
     del flush
     torch.cuda.empty_cache()
-    peak = measure_fp32_peak(torch, dev)
+    mma = int(sc.p_of_sphere().max()) <= 31
+    peak = measure_fp64_peak(torch, dev) if mma else measure_fp32_peak(torch, dev)
     flops = algorithmic_flops(sc)
     t32 = float(np.mean(ms32))
     achieved = flops / (t32 * 1e-3) / 1e12
     line = {
         "metric": METRIC, "value": 1e3 / float(np.mean(ms)), "unit": "solves/s", "n_gpus": 1, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": float(np.mean(ms)), "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "f32 translations, f64 residuals", "data": "synthetic",
+        "vs_baseline": None, "dtype": "f64" if mma else "f32 translations, f64 residuals", "data": "synthetic",
         "config": {"workload": sc.name + " mixed precision", "gmres_restart": sc.gmres_restart,
                    "gmres_tolerance": sc.gmres_tolerance,
-                   "fp32_pair_tables": "tcgen05 kind::tf32 3xTF32 products (k_pair_tc), built once per handle "
-                                       "before the timed solves; inside the e2e leg",
+                   "arnoldi_operator": "FP64 tensor cores" if mma else "FP32 CUDA cores",
+                   "pair_tables": "built once per handle before the timed solves; inside the e2e leg",
                    "l2": "Krylov basis exceeds L2; 256 MB L2 flush between steps"},
         "fp64": {"ms_per_solve": st64["ms_total"], "iterations": st64["iterations"],
                  "ms_per_operator": ms64_per_mv},
         "iterations": its[-1], "matvecs": mvs[-1], "backward_error": st["backward_error"],
         "rel_coefficient_error": float(np.linalg.norm(x - x64) / np.linalg.norm(x64)),
         "c_ext_rel_error": float(abs(c[1] - c64[1]) / abs(c64[1])),
-        "roofline": {"bound": "fp32", "compute": "FP32 CUDA-core pipe (FFMA); no tensor-core instruction",
+        "roofline": {"bound": "fp64" if mma else "fp32",
+                     "compute": "FP64 tensor cores (mma.sync f64)" if mma else "FP32 CUDA-core pipe (FFMA)",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                     "frac": achieved / peak, "traffic": None, "kernel": "k_direct<cplxf> (+k_direct_finish)",
+                     "frac": achieved / peak, "traffic": None, "kernel": ("k_direct_mma" if mma else "k_direct<cplxf>") + " (+k_direct_finish)",
                      "flops_per_launch": flops, "ms_per_launch": t32,
-                     "peak_source": "cuBLAS FP32 SGEMM 8192^3 (TF32 off) measured in this run (no FP32 figure "
+                     "peak_source": ("cuBLAS FP64 DGEMM 8192^3" if mma else "cuBLAS FP32 SGEMM 8192^3 (TF32 off)") +
+                                    " measured in this run (no such figure "
                                     "in MEASURED_PEAKS.json)"},
         "e2e": {"value": 1e3 / e2e_ms, "unit": "solves/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(xh.nbytes)},
@@ -926,11 +932,11 @@ def main():
             "latency_ms": {"p50": percentile(lat, 50), "p99": percentile(lat, 99)},
             "solve": {"iterations": iters, "matvecs_per_solve": mv_count // args.steps,
                       "backward_error": berr, "ms_operator_per_solve": mv_ms / args.steps},
-            "roofline": {"bound": "fp64", "compute": "FP64 CUDA-core pipe (DFMA); no tensor-core instruction",
+            "roofline": {"bound": "fp64", "compute": "FP64 tensor cores (mma.sync f64; above order 31 DFMA)",
                          "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak, "traffic": traffic,
-                         "kernel": ("k_translate (ML-FMM passes) + k_direct_finish" if fmm
-                                    else "k_direct (+k_direct_finish)"), "flops_per_launch": flops,
+                         "kernel": ("k_translate_mma, k_translate (ML-FMM passes) + k_direct_finish" if fmm
+                                    else "k_direct_mma (+k_direct_finish)"), "flops_per_launch": flops,
                          "ms_per_launch": avg_mv,
                          "peak_source": "cuBLAS FP64 DGEMM 8192^3 measured in this run (no FP64 figure in "
                                         "MEASURED_PEAKS.json)"},

@@ -97,8 +97,8 @@ typedef struct foggy_params {
                                     and box coefficients), the true residual at the start and
                                     at every restart in FP64, so the restarts refine to
                                     gmres_tolerance.  foggy_matvec stays FP64.  Where the
-                                    FP64 operator runs on the tensor cores (pair tables kept,
-                                    orders up to 31) it is as fast, and the Arnoldi steps of
+                                    FP64 operator runs on the tensor cores (orders up to 31;
+                                    blocks: with pair tables) it is as fast, and the Arnoldi steps of
                                     the direct operator use it instead                      */
 } foggy_params;
 

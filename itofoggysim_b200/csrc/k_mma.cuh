@@ -24,7 +24,7 @@
 // mma.sync f64 runs at the FP64 pipe's full rate here (measured 64 FMA per clock and SM from four warps with one
 // chain each), so the products themselves take a quarter of the time; the rest is forming w, the phases and
 // the loads around them (L1 data pipe half busy, instruction fetch where the code outgrows its cache).
-// One application: 1000 lognormal spheres (orders 11..28) 47.8 -> 22.0 ms, 64 spheres of order 15
+// One application: 1000 lognormal spheres (orders 11..28) 47.8 -> 21.4 ms, 64 spheres of order 15
 // 0.222 -> 0.111 ms, 40 of order 5 78 -> 47 us (k_direct before, this after; copies included).
 #pragma once
 
