@@ -6,8 +6,8 @@
 // the product library calls into it.
 //
 // Every function cites the reference file:line it follows (paths relative to the reference
-// project root).  The Wigner-3j symbols come from the reference's own C library wigxjpf 1.10
-// (wigxjpf_1_10/src), compiled from its sources into oracle/_ref/ by oracle/Makefile.
+// project root).  The Wigner-3j symbols, which the reference takes from the C library wigxjpf, come from a recurrence
+// in extended precision here; tests/test_oracle_wigner.py holds them against exact rational arithmetic.
 //
 // Conventions (identical to the reference):
 //   * complex numbers are two interleaved doubles (Fortran complex(8));
@@ -26,25 +26,6 @@
 #include <map>
 #include <array>
 #include <omp.h>
-
-extern "C" {
-void wig_table_init(int max_two_j, int wigner_type);
-void wig_thread_temp_init(int max_two_j);
-void wig_temp_free(void);
-double wig3jj(int two_j1, int two_j2, int two_j3, int two_m1, int two_m2, int two_m3);
-}
-
-// wigxjpf keeps one scratch array per thread (wig_thread_temp_init allocates a new one each call).
-// Grow the calling thread's array when it is smaller than asked, never shrink it: the main thread
-// also runs in the OpenMP regions below, and a smaller array left there would make a later 3j call
-// of higher degree on that thread fail.
-static void ensure_wig_temp(int max_two_j) {
-    static thread_local int have = -1;
-    if (have >= max_two_j) return;
-    if (have >= 0) wig_temp_free();
-    wig_thread_temp_init(max_two_j);
-    have = max_two_j;
-}
 
 typedef std::complex<double> cd;
 static const double PI = 3.14159265358979323846264338327950288;
@@ -248,10 +229,73 @@ void pi_tau_table(double theta, int nmax, int cs_phase, double* pi, double* tau)
 }
 
 // ------------------------------------------------------------------------------------------
-// Wigner 3j through the reference's wigxjpf (libmath/src/math/lib_math_wigner.f90:45-72)
+// Wigner 3j (libmath/src/math/lib_math_wigner.f90:45-72)
 // ------------------------------------------------------------------------------------------
-inline double w3j(int j1, int j2, int j3, int m1, int m2, int m3) {
-    return wig3jj(2 * j1, 2 * j2, 2 * j3, 2 * m1, 2 * m2, 2 * m3);
+// All j3 of (j1 j2 j3; m1 m2 -m1-m2) at once, in extended precision, by the three-term recurrence in j3 of
+// K. Schulten and R. G. Gordon, J. Math. Phys. 16, 1961 (1975), eqs. 5-8:
+//   j A(j+1) f(j+1) + B(j) f(j) + (j+1) A(j) f(j-1) = 0,
+// from both ends (each side is the growing one there), joined inside the classically allowed range, where neither
+// direction loses accuracy; the scale is sum (2j+1) f^2 = 1 and the sign f(j1+j2) (-1)^(j1-j2+m1+m2) > 0.
+struct Wigner3jFamily {
+    int j1 = -1, j2 = 0, m1 = 0, m2 = 0, lo = 0;
+    std::vector<double> f;   // j3 = lo ..
+    std::vector<long double> A, B, F, G;
+
+    void make(int j1_, int j2_, int m1_, int m2_) {
+        j1 = j1_; j2 = j2_; m1 = m1_; m2 = m2_;
+        const int m3 = -m1 - m2, hi = j1 + j2;
+        lo = std::max(std::abs(j1 - j2), std::abs(m3));
+        const int n = hi - lo + 1;
+        f.assign(n, 0.0);
+        A.assign(n + 1, 0.0L);
+        B.assign(n, 0.0L);
+        F.assign(n, 0.0L);
+        G.assign(n, 0.0L);
+        // A(j) / j, A(j + 1) / (j + 1) and B(j) / (j (j + 1)): finite at j = 0 too, where j1 = j2 and m3 = 0
+        for (int i = 0; i <= n; ++i) {
+            const long double j = lo + i, d = j1 - j2, t = hi + 1;
+            if (lo + i > 0) A[i] = std::sqrt((j - d) * (j + d) * (t - j) * (t + j) * (j - m3) * (j + m3)) / j;
+        }
+        for (int i = 0; i < n; ++i) {
+            const long double j = lo + i;
+            const long double c = (long double)m3 * ((long double)j1 * (j1 + 1) - (long double)j2 * (j2 + 1));
+            B[i] = -(2 * j + 1) * ((lo + i > 0 ? c / (j * (j + 1)) : 0.0L) - (m2 - m1));
+        }
+        F[0] = 1.0L;
+        for (int i = 0; i + 1 < n; ++i) F[i + 1] = -(B[i] * F[i] + (i > 0 ? A[i] * F[i - 1] : 0.0L)) / A[i + 1];
+        G[n - 1] = 1.0L;
+        for (int i = n - 1; i > 0; --i) G[i - 1] = -(B[i] * G[i] + (i + 1 < n ? A[i + 1] * G[i + 1] : 0.0L)) / A[i];
+        // the most oscillating place: 4 A(j) A(j+1) - B(j)^2 in the units of A
+        int s = 0;
+        long double best = -1e300L;
+        for (int i = 0; i < n; ++i) {
+            const long double a = A[i] * A[i + 1], v = 4.0L - (a > 0.0L ? B[i] * B[i] / a : 1e300L);
+            if (v > best) {
+                best = v;
+                s = i;
+            }
+        }
+        const int e = std::min(s + 1, n - 1);
+        const long double scale = (F[s] * G[s] + F[e] * G[e]) / (G[s] * G[s] + G[e] * G[e]);
+        for (int i = s + 1; i < n; ++i) F[i] = scale * G[i];
+        long double sum = 0.0L;
+        for (int i = 0; i < n; ++i) sum += (2 * (lo + i) + 1) * F[i] * F[i];
+        const bool neg = ((j1 - j2 + m1 + m2) & 1) != 0;
+        const long double r = ((F[n - 1] < 0.0L) != neg ? -1.0L : 1.0L) / std::sqrt(sum);
+        for (int i = 0; i < n; ++i) f[i] = (double)(r * F[i]);
+    }
+};
+
+static inline double w3j(int j1, int j2, int j3, int m1, int m2, int m3) {
+    if (m1 + m2 + m3 != 0 || std::abs(m1) > j1 || std::abs(m2) > j2 || std::abs(m3) > j3) return 0.0;
+    if (j3 < std::abs(j1 - j2) || j3 > j1 + j2) return 0.0;
+    const bool zero = m1 == 0 && m2 == 0;
+    if (zero && ((j1 + j2 + j3) & 1)) return 0.0;
+    // the translation coefficients walk j3 with the orders fixed, and need orders 0 beside them
+    static thread_local Wigner3jFamily last[2];
+    Wigner3jFamily& w = last[zero];
+    if (w.j1 != j1 || w.j2 != j2 || w.m1 != m1 || w.m2 != m2) w.make(j1, j2, m1, m2);
+    return w.f[j3 - w.lo];
 }
 
 // lib_math_vector_spherical_harmonics.f90:2235-2261
@@ -310,7 +354,6 @@ void translation_xu(double x, double theta, double phi, int n1, int n2, int nu1,
     int cnt_nu = (nu2 + 1) * (nu2 + 1) - nu1 * nu1;
 #pragma omp parallel
     {
-        ensure_wig_temp(2 * (2 * pmax + 2));
 #pragma omp for schedule(dynamic)
         for (int n = n1; n <= n2; ++n) {
             for (int m = -n; m <= n; ++m) {
@@ -789,7 +832,6 @@ void matvec_direct(Problem& P, const cd* x, cd* y, int j0 = 0, int j1 = -1, bool
     for (int w = 0; w < (int)work.size(); ++w) {
         int j = work[w].first;
         std::vector<cd> lA, lB;
-        ensure_wig_temp(2 * (4 * P.n2 + 8));
         int ip = P.pidx[j];
         int a0 = P.nr[2 * ip];
         cd* yj = y + (size_t)2 * C * j;
@@ -945,12 +987,6 @@ GmresOut gmres(Op op, size_t n, const cd* b, cd* x, int restart, double tol, int
 // C API used by tests/ (through ctypes), __graft_entry__.smoke() and bench.py's CPU baseline
 // ==========================================================================================
 extern "C" {
-
-void orc_init(int max_n) {
-    int two_j = 2 * (4 * max_n + 8);
-    wig_table_init(two_j, 3);
-    ensure_wig_temp(two_j);
-}
 
 int orc_sph_jn(double x, int nmax, double* out) { sph_jn(x, nmax, out); return 0; }
 int orc_sph_yn(double x, int nmax, double* out) { sph_yn(x, nmax, out); return 0; }
@@ -1294,7 +1330,6 @@ struct Fmm {
         if (it == cache.end()) {
             int cr = (r2 + 1) * (r2 + 1) - r1 * r1, cc = (c2 + 1) * (c2 + 1) - c1 * c1;
             std::vector<cd> A((size_t)cr * cc), B((size_t)cr * cc);
-            ensure_wig_temp(2 * (4 * std::max(std::max(r2, c2), P.n2) + 8));
             translation_xu(rho, th, ph, r1, r2, c1, c2, z, A.data(), B.data());
             it = cache.emplace(key, std::make_pair(std::move(A), std::move(B))).first;
         }
@@ -1537,7 +1572,6 @@ int orc_pairs_apply(void* p, const double* xin, int npairs, const int* pj, const
     int C = P->cnt();
 #pragma omp parallel for schedule(dynamic)
     for (int w = 0; w < npairs; ++w) {
-        ensure_wig_temp(2 * (4 * P->n2 + 8));
         int j = pj[w], l = pl[w];
         if (j == l) continue;
         int ja, jb, la, lb;

@@ -1,8 +1,7 @@
 """ctypes wrapper of the FP64 CPU oracle (test infrastructure only).
 
 Only tests/, __graft_entry__.smoke() and the CPU-baseline leg of bench.py import this module.
-It loads oracle/liboracle.so, which restates the reference algorithms (see oracle.cpp) and
-links the reference's own wigxjpf library built into oracle/_ref/.
+It loads oracle/liboracle.so, which restates the reference algorithms (see oracle.cpp).
 """
 import ctypes as C
 import os
@@ -19,15 +18,8 @@ lp = np.ctypeslib.ndpointer(dtype=np.int64, flags="C_CONTIGUOUS")
 
 
 def build():
-    """Compile liboracle.so (and _ref/libwigxjpf.a from the reference checkout named by the
-    environment variable FOGGY_REFERENCE; without it the prebuilt _ref/ library is used)."""
-    ref = os.environ.get("FOGGY_REFERENCE", "")
-    args = ["make", "-s", "-C", HERE]
-    if ref and os.path.isdir(ref):
-        args.append("REF=" + ref)
-    elif not os.path.exists(os.path.join(HERE, "_ref", "libwigxjpf.a")):
-        raise RuntimeError("oracle/_ref/libwigxjpf.a is missing: set FOGGY_REFERENCE to the reference checkout")
-    subprocess.run(args, check=True)
+    """Compile liboracle.so when oracle.cpp is newer."""
+    subprocess.run(["make", "-s", "-C", HERE], check=True)
 
 
 def lib():
@@ -35,10 +27,9 @@ def lib():
     if _LIB is not None:
         return _LIB
     path = os.path.join(HERE, "liboracle.so")
-    if not os.path.exists(path):
+    if not os.path.exists(path) or os.path.getmtime(path) < os.path.getmtime(os.path.join(HERE, "oracle.cpp")):
         build()
     L = C.CDLL(path)
-    L.orc_init.argtypes = [C.c_int]
     L.orc_sph_jn.argtypes = [C.c_double, C.c_int, dp]
     L.orc_sph_yn.argtypes = [C.c_double, C.c_int, dp]
     L.orc_legendre_table.argtypes = [C.c_double, C.c_int, dp]
@@ -69,7 +60,6 @@ def lib():
     L.orc_solve.argtypes = [C.c_void_p, dp, dp, C.c_int, C.c_double, C.c_int, C.c_void_p,
                             ip, C.POINTER(C.c_double)]
     L.orc_cross_sections.argtypes = [C.c_void_p, dp, dp]
-    L.orc_init(64)
     _LIB = L
     return L
 
