@@ -43,10 +43,12 @@ struct Trace {
     Trace& operator=(const Trace&) = delete;
 };
 
-// The tensor-core operator's launches for a number of vectors, one per kernel class, and the slabs they fill.
+// The tensor-core operator's launches, one per kernel class, and the slabs they fill: how each target's sources are split
+// into CTAs, by use (one vector with a slab per source bucket; one vector; one of several) and by whether S is summed.
+enum MmaUse { kMmaStatic, kMmaSingle, kMmaBlock, kMmaUses };
 struct MmaPlan {
     struct Launch {
-        int first, count, ctas, pp;   // shares work[first .. first + count - 1]
+        int first, count, ctas, pp;   // shares work[first .. first + count - 1], CTAs per vector
     };
     std::vector<Launch> launches;
     MmaWork* d_work = nullptr;
@@ -115,7 +117,7 @@ struct foggy_handle_s {
     int K = 0;
     // operator launches: (target bucket, source bucket) pairs of truncation-order buckets
     std::vector<DirectBucket> launches_direct;
-    std::map<std::pair<int, bool>, MmaPlan> mma_plans;   // the tensor-core operator's, by vectors and no tables
+    MmaPlan mma_plans[kMmaUses][2];   // the tensor-core operator's, without and with S summed
     int* d_bucket_lists = nullptr;
     int nbuckets = 0, cmax = 1;
     // waves and right-hand side
@@ -550,7 +552,8 @@ static_assert(kBucketBounds[kNumBounds - 1] >= kMaxDegree, "every order needs a 
 // Truncation-order buckets of the spheres and the (target bucket, source bucket) launches of
 // the direct operator.  Bucket upper bounds grow in steps of 4 degrees; each launch gets enough
 // CTAs per target to fill the GPU.
-int mma_plan(foggy_handle h, int nrhs, bool sum, const MmaPlan** out);
+int make_mma_plan(foggy_handle h, MmaUse use, bool sum, MmaPlan& p);
+void free_mma_plans(foggy_handle h);
 int plan_direct(foggy_handle h) {
     const int* bounds = kBucketBounds;
     std::vector<std::vector<int>> members;
@@ -598,14 +601,23 @@ int plan_direct(foggy_handle h) {
             b.pp = std::max(bp[t], bp[s]);
             h->launches_direct.push_back(b);
         }
-    // the plans of single vectors, so that no later call allocates for them
-    const MmaPlan* plan = nullptr;
-    for (int i = 0; i < 4; ++i) TRY(mma_plan(h, i & 1, (i & 2) != 0, &plan));
+    // made here, so that no later call allocates for them
+    free_mma_plans(h);
+    for (int u = 0; u < kMmaUses; ++u)
+        for (int sum = 0; sum < (u == kMmaBlock ? 1 : 2); ++sum)   // blocks without tables run on the CUDA cores
+            TRY(make_mma_plan(h, (MmaUse)u, sum != 0, h->mma_plans[u][sum]));
     return FOGGY_OK;
 }
 
-// The tensor-core operator's plan for nrhs vectors at a time (each has its own slabs), over the pair tables or summing S (sum); nrhs = 0: one
-// vector with one slab per source bucket (foggy_matvec_static).
+// A block's vectors are split as four of them at once would want: by the scene alone, not by how many vectors a launch
+// happens to hold, so that a vector's sums are the same bits whatever else is in the block and however many of its
+// vectors have converged and left.  More CTAs than many vectors need cost their set-up, fewer leave SMs idle when
+// the last few vectors remain; 64 spheres of order 15 get 4 batches a CTA, where one vector wants 3 and 32 want 16.
+// With splits by the count of vectors 32 solves of them took 98.0 ms and 12 applications of 130 spheres 25.8 ms, with
+// these 97.3 and 26.1 (the runs of either differ by 1 and 5 %).
+constexpr int kMmaBlockVectors = 4;
+
+// The tensor-core operator's plan of a use.
 //
 // All (target bucket, source bucket) shares of a kernel class are one launch, largest degrees first, so that buckets of a
 // few spheres fill the GPU together, and the next class's CTAs start while the last of a class run out.  One launch a
@@ -613,11 +625,9 @@ int plan_direct(foggy_handle h) {
 // application, 1000 27.3 -> 24.0 ms, 8 spheres 108 -> 76 us.  The shares' CTAs take about the
 // same number of batches B of four translations, the B that ends first, a CTA costing its batches plus 0.3 of one for
 // its set-up, larger degrees more by their square.  Slabs bound the chunks.
-int make_mma_plan(foggy_handle h, int nrhs, bool sum, MmaPlan& p) {
-    const int nb = h->nbuckets, nv = std::max(1, nrhs), per = nrhs == 0 ? 1 : std::max(1, h->cmax / nv);
+int make_mma_plan(foggy_handle h, MmaUse u, bool sum, MmaPlan& p) {
+    const int nb = h->nbuckets, nv = u == kMmaBlock ? kMmaBlockVectors : 1, per = u == kMmaStatic ? 1 : h->cmax;
     p.use.nb = nb;
-    p.use.per_bucket = per;
-    p.use.per_rhs = nb * per;
     std::vector<MmaWork> work;
     for (int cls = 4; cls >= 0; --cls) {
         std::vector<int> in;
@@ -659,12 +669,16 @@ int make_mma_plan(foggy_handle h, int nrhs, bool sum, MmaPlan& p) {
         for (int i : in) {
             const DirectBucket& b = h->launches_direct[i];
             const int t = i / nb, s = i % nb, c = chunks_for(i, bestB);
-            work.push_back(MmaWork{b.targets, b.sources, b.ntargets, b.nsources, s * per, c, b.pp, mma_unit_size(b.pp), l.ctas});
+            // the source bucket for now, its first slab below
+            work.push_back(MmaWork{b.targets, b.sources, b.ntargets, b.nsources, s, c, b.pp, mma_unit_size(b.pp), l.ctas});
             p.use.c[t][s] = (unsigned char)c;
-            l.ctas += b.ntargets * nv * c;
+            p.use.per_bucket = std::max(p.use.per_bucket, c);
+            l.ctas += b.ntargets * c;
         }
         p.launches.push_back(l);
     }
+    for (MmaWork& w : work) w.slab *= p.use.per_bucket;
+    p.use.per_rhs = nb * p.use.per_bucket;
     // compact bucket of each step of four orders
     int id = 0;
     for (int q = 0; q < 12; ++q) {
@@ -677,16 +691,12 @@ int make_mma_plan(foggy_handle h, int nrhs, bool sum, MmaPlan& p) {
     return FOGGY_OK;
 }
 
-int mma_plan(foggy_handle h, int nrhs, bool sum, const MmaPlan** out) {
-    const auto key = std::make_pair(nrhs, sum);
-    auto it = h->mma_plans.find(key);
-    if (it == h->mma_plans.end()) {
-        MmaPlan p;
-        TRY(make_mma_plan(h, nrhs, sum, p));
-        it = h->mma_plans.emplace(key, std::move(p)).first;
-    }
-    *out = &it->second;
-    return FOGGY_OK;
+void free_mma_plans(foggy_handle h) {
+    for (auto& by_use : h->mma_plans)
+        for (MmaPlan& p : by_use) {
+            dfree(h, p.d_work);
+            p = MmaPlan{};
+        }
 }
 
 // The pair tables over groups of pairs (k_pair_tables.cu).  The pairs are grouped by
@@ -1442,13 +1452,11 @@ int apply_operator_fmm(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false
     return FOGGY_OK;
 }
 
-// Y_r = A X_r on the tensor cores for the nrhs vectors X + r n_unk (nrhs = 0: foggy_matvec_static's one); a.partial
-// holds the plan's slabs.  xref given: one vector, Y and xref in the reference layout.
-int launch_mma(foggy_handle h, DirectArgs a, int nrhs, const cplx* X, cplx* Y, const cplx* xref = nullptr) {
-    const MmaPlan* p = nullptr;
-    TRY(mma_plan(h, nrhs, a.pt.stab == nullptr, &p));
+// Y_r = A X_r on the tensor cores for the nv vectors X + r n_unk; a.partial holds the plan's slabs for each.  xref given:
+// one vector, Y and xref in the reference layout.
+int launch_mma(foggy_handle h, DirectArgs a, MmaUse u, int nv, const cplx* X, cplx* Y, const cplx* xref = nullptr) {
+    const MmaPlan* p = &h->mma_plans[u][a.pt.stab == nullptr];
     const MmaTabs mt = mma_tabs(h);
-    const int nv = std::max(1, nrhs);
     a.x = X;
     for (const MmaPlan::Launch& l : p->launches)
         launch_direct_mma(a, mt, p->d_work + l.first, l.count, l.ctas, l.pp, nv, h->n_unk, p->use.per_rhs,
@@ -1474,7 +1482,7 @@ int apply_operator(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false) {
     a.fp32 = (!mma && fp32 && h->stab32_ready) ? 1 : 0;
     Trace tr(a.fp32 ? "operator (FP32)" : "operator (FP64)");
     if (mma) {
-        TRY(launch_mma(h, a, 1, x, y));
+        TRY(launch_mma(h, a, kMmaSingle, 1, x, y));
     } else {
         for (const DirectBucket& b : h->launches_direct) launch_direct(a, b, h->stream);
         CKL(h);
@@ -1555,8 +1563,7 @@ void free_scene(foggy_handle h) {
     dfree(h, h->d_partial);
     dfree(h, h->d_bslab);
     h->bslab_vectors = 0;
-    for (auto& [key, p] : h->mma_plans) dfree(h, p.d_work);
-    h->mma_plans.clear();
+    free_mma_plans(h);
     dfree(h, h->d_stab);
     dfree(h, h->d_stab32);
     h->stab32_ready = false;
@@ -2175,7 +2182,7 @@ int32_t foggy_matvec(foggy_handle h, const double* x, double* y, int32_t mem) {
         const DirectArgs a = direct_args(h, h->d_tmp_in);
         packed = mma_operator(h, a);
         Trace tr("operator (FP64)");
-        if (packed) TRY(launch_mma(h, a, 1, h->d_tmp_in, yr, xr));
+        if (packed) TRY(launch_mma(h, a, kMmaSingle, 1, h->d_tmp_in, yr, xr));
     }
     if (!packed) {
         TRY(apply_operator(h, h->d_tmp_in, h->d_tmp_out));
@@ -2807,7 +2814,7 @@ extern "C" int32_t foggy_matvec_static(foggy_handle h, const double* x, double* 
     a.partial = partial;
     a.cmax = 1;
     if (mma_operator(h, a)) {
-        TRY(launch_mma(h, a, 0, xin, yout));
+        TRY(launch_mma(h, a, kMmaStatic, 1, xin, yout));
     } else {
         for (const DirectBucket& b : h->launches_direct) {
             DirectBucket b1 = b;
@@ -2945,8 +2952,9 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
     }
     TRY(ensure_pair_tables(h, must32));
     const BlockArgs ba = block_args(h, X, Y, nrhs, fp32);
-    // without tables the CUDA-core kernel sums S once for a tile of vectors
-    if (!must32 && mma_operator(h, ba.d) && (ba.d.pt.stab || (nrhs == 1 && !(fp32 && ba.d.pt.stab32)))) {
+    // without tables the CUDA-core kernel sums S once for a tile of vectors (for one too: a block's last vector keeps the
+    // operator that it had beside the others)
+    if (!must32 && mma_operator(h, ba.d) && ba.d.pt.stab) {
         // One vector per CTA: a batch's set-up that vectors could share is small beside its products, and the pair's
         // coaxial block comes from L2 after the first.  83 spheres, 5 right-hand sides to 1e-6: 161 -> 55 ms a request
         // (the tile autotuner's runs are gone too).  As many vectors at a time as have slabs: the handle's own, or a
@@ -2954,8 +2962,9 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
         // together (64 spheres, 32 vectors: 14 + 14 + 4 vectors took 9 waves of 296 CTAs, 32 take 7).
         Trace tr("block operator (FP64)");
         DirectArgs a = ba.d;
-        int most = h->cmax;
-        const size_t one = (size_t)h->nbuckets * h->n_unk;
+        const SlabUse& use = h->mma_plans[kMmaBlock][0].use;
+        int most = std::max(1, h->nbuckets * h->cmax / std::max(1, use.per_rhs));
+        const size_t one = (size_t)use.per_rhs * h->n_unk;
         // at most a quarter of what the budget leaves: a tight one is for the calls to come
         const size_t room = (h->budget > h->bytes_in_use ? h->budget - h->bytes_in_use : 0) +
                             (size_t)h->bslab_vectors * one * sizeof(cplx);
@@ -2973,7 +2982,7 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
         const int groups = (nrhs + most - 1) / most, per = (nrhs + groups - 1) / groups;
         for (int r = 0; r < nrhs; r += per) {
             const int nr = std::min(per, nrhs - r);
-            TRY(launch_mma(h, a, nr, X + (size_t)r * h->n_unk, Y + (size_t)r * h->n_unk));
+            TRY(launch_mma(h, a, kMmaBlock, nr, X + (size_t)r * h->n_unk, Y + (size_t)r * h->n_unk));
         }
         CKL(h);
         return FOGGY_OK;
@@ -3413,7 +3422,7 @@ int32_t foggy_block_tiles(foggy_handle h, int32_t precision, int32_t nrhs, int32
         const DirectBucket& b = h->launches_direct[i];
         int R = 0;
         // one vector per CTA on the tensor cores
-        if (!ba.d.fp32 && mma_operator(h, ba.d) && (tabs || nrhs == 1)) R = 1;
+        if (!ba.d.fp32 && mma_operator(h, ba.d) && tabs) R = 1;
         else rc = choose_tile(h, ba, b, tabs, &R);
         out[4 * i] = b.ntargets;
         out[4 * i + 1] = b.nsources;

@@ -148,8 +148,8 @@ void build_mma_tables(int pmax, const std::vector<double>& delta, std::vector<do
 int mma_ctas_per_sm(int pp, bool sum);
 // the kernel instantiation of a largest degree, 0..4: launches of one class go as one
 int mma_class(int pp, bool sum);
-// A (target bucket, source bucket) share of a launch: CTAs cta0 .. cta0 + ntargets nrhs chunks - 1, vector fastest, then
-// target, then chunk
+// A (target bucket, source bucket) share of a launch: per vector CTAs cta0 .. cta0 + ntargets chunks - 1, target fastest,
+// then chunk; a CTA's vectors follow one another in the grid
 struct MmaWork {
     const int* targets;
     const int* sources;
@@ -159,7 +159,7 @@ struct MmaWork {
     int cta0;
 };
 int mma_unit_size(int pp);
-// nw shares of one class, largest degree pp, `ctas` CTAs in all; without a.pt.stab S is summed; vectors a.x + r ld.  after_other: the
+// nw shares of one class, largest degree pp, `ctas` CTAs a vector; without a.pt.stab S is summed; vectors a.x + r ld.  after_other: the
 // launch before it on the stream is one of these with the same input, and may still be running out
 void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const MmaWork* w, int nw, int ctas, int pp, int nrhs,
                        int64_t ld, int per_rhs, bool after_other, cudaStream_t s);

@@ -146,15 +146,16 @@ __global__ void __launch_bounds__(32 * W, CTAS) k_direct_mma(DirectArgs a, MmaTa
     // the next class's CTAs may start once all of these have (they fill other slabs); each launch ends after the one before
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const SceneView& sc = a.sc;
+    // right-hand side fastest: the CTAs that read one pair's coaxial block run together
+    const int rhs = blockIdx.x % nrhs, unit = blockIdx.x / nrhs;
     // this CTA's share: the last one that starts no later (every warp looks, one load per lane and 32 shares)
     int at = -1;
     for (int b = 0; b < nw; b += 32) {
         const int i = b + (threadIdx.x & 31);
-        at += __popc(__ballot_sync(0xffffffffu, i < nw && work[i].cta0 <= (int)blockIdx.x));
+        at += __popc(__ballot_sync(0xffffffffu, i < nw && work[i].cta0 <= unit));
     }
     const MmaWork bk = work[at];
-    // right-hand side fastest: the CTAs that read one pair's coaxial block run together
-    const int id = blockIdx.x - bk.cta0, rhs = id % nrhs, tc = id / nrhs, c = tc / bk.ntargets;
+    const int tc = unit - bk.cta0, c = tc / bk.ntargets;
     const int j = bk.targets[tc % bk.ntargets];
     if (!sc.couple[j]) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -225,7 +226,7 @@ void launch_direct_mma(const DirectArgs& a, const MmaTabs& mt, const MmaWork* w,
     auto go = [&](auto* kernel, int warps, size_t smem) {
         raise_smem_ceiling(reinterpret_cast<const void*>(kernel), smem);
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)ctas);
+        cfg.gridDim = dim3((unsigned)ctas * nrhs);
         cfg.blockDim = dim3(32 * warps);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
