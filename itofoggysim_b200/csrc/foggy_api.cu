@@ -2280,12 +2280,14 @@ int32_t foggy_get_field(foggy_handle h, const double* x, int32_t mem, int32_t np
     // per-call buffers: sphere radii, and the points and fields when they live on the host
     void* tmp = nullptr;
     const size_t np = (size_t)npoints;
-    size_t bytes = (rad.size() + 1) / 2 * 2 * sizeof(double) + len * sizeof(cplx);
+    const size_t n_part = field_part(h->N, h->pg, npoints);
+    size_t bytes = (rad.size() + 1) / 2 * 2 * sizeof(double) + len * sizeof(cplx) + n_part * sizeof(double);
     if (mem == FOGGY_MEM_HOST) bytes += len * sizeof(cplx) + 3 * np * sizeof(double) + 6 * np * sizeof(cplx);
     CK(h, talloc(h, &tmp, bytes));
     double* d_rad = static_cast<double*>(tmp);
     cplx* d_ab = reinterpret_cast<cplx*>(d_rad + (rad.size() + 1) / 2 * 2);
-    char* q = reinterpret_cast<char*>(d_ab + len);
+    double* d_part = reinterpret_cast<double*>(d_ab + len);
+    char* q = reinterpret_cast<char*>(d_part + n_part);
     cudaError_t e = cudaMemcpyAsync(d_rad, rad.data(), rad.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream);
     if (mem == FOGGY_MEM_HOST) {
         cplx* xs = reinterpret_cast<cplx*>(q);
@@ -2299,16 +2301,8 @@ int32_t foggy_get_field(foggy_handle h, const double* x, int32_t mem, int32_t np
         pd = ps;
     }
     if (e == cudaSuccess) {
-        // warps per CTA: enough for 16 on every SM, no more than there are spheres or shared memory for
-        const int blocks = (npoints + 31) / 32;
-        int warps = std::max(1, std::min({16, h->N, (148 * 16 + blocks - 1) / blocks}));
-        warps = std::max(warps, std::min(4, h->N));
-        while (warps > 1 && field_smem_bytes(h->pg, 32 * warps) > ((size_t)200 << 10)) --warps;
-        const size_t smem = field_smem_bytes(h->pg, 32 * warps);
-        raise_smem_ceiling(reinterpret_cast<const void*>(k_field), smem);
-        k_field_coeff<<<h->N, 128, 0, h->stream>>>(C, xd, d_ab);
-        k_field<<<blocks, 32 * warps, smem, h->stream>>>(scene_view(h), d_rad, h->pg, C, d_ab, npoints, pd, e_field_0,
-                                                         h->prm.n_medium / 299792458.0, ed, hd);
+        launch_field(scene_view(h), d_rad, h->pg, C, xd, d_ab, npoints, pd, e_field_0, h->prm.n_medium / 299792458.0, ed, hd,
+                     d_part, h->stream);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && mem == FOGGY_MEM_HOST) {

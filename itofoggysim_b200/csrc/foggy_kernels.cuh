@@ -47,12 +47,11 @@ __global__ void k_unpack(SceneView sc, int pg, const double* g, const cplx* xref
 __global__ void k_pack(SceneView sc, int pg, const double* g, const cplx* ydev, const cplx* identity_ref,
                        cplx* yref);
 __global__ void k_cross_sections(SceneView sc, const cplx* x, const cplx* pq, double* part);
-// scattered E, H at points from the coefficients that k_field_coeff scaled (reference layout x, C entries per part
-// and sphere -> ab, a and b of an order side by side); 32 points per CTA, any number of warps up to 16
-__global__ void k_field_coeff(int C, const cplx* x, cplx* ab);
-__global__ void k_field(SceneView sc, const double* radius_s, int pg, int C, const cplx* ab, int npoints,
-                        const double* pts, double e0, double h_factor, cplx* E_out, cplx* H_out);
-size_t field_smem_bytes(int pg, int threads);
+// scattered E, H at points (reference layout coefficients x, C entries per part and sphere; ab: 2 C N entries and part:
+// field_part doubles of scratch)
+size_t field_part(int n, int pg, int npoints);
+void launch_field(const SceneView& sc, const double* radius_s, int pg, int C, const cplx* x, cplx* ab, int npoints,
+                  const double* pts, double e0, double h_factor, cplx* E_out, cplx* H_out, double* part, cudaStream_t s);
 
 // k_direct.cu -- all-pairs sphere coupling (the direct operator)
 // Tables of the Wigner small-d recurrence (degrees <= K).
