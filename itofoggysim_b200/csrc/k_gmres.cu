@@ -116,11 +116,15 @@ __global__ void k_update_x(cplx* x, const cplx* V, int64_t ld, const cplx* y, in
 
 // ---- one Arnoldi step's orthogonalisation --------------------------------------------------------
 // Classical Gram-Schmidt twice, the norm and the Givens rotation, for one Krylov space or one per slot
-// (blockIdx.y), as three launches: dots | subtract, dots again | subtract, norm, Givens.  Each block owns a slice
-// of w; the last block to finish (an atomic ticket, no waiting) adds the blocks' partial sums in block order, so a
-// result does not depend on the order of arrival or on the other slots.  Launch-bound on small problems: the eight launches
-// before, one thread for the Givens column, against these four: a solve of 32640 unknowns in 25 steps 4.91 -> 4.43 ms; on
-// large ones the basis is read three times a step instead of four.
+// (blockIdx.y), as three launches and a fourth that scales: dots | subtract, dots again | subtract, norm, Givens | next
+// vector.  Each block owns a slice of w; the last block to finish (an atomic ticket, no waiting) adds the blocks' partial
+// sums in block order, so a result does not depend on the order of arrival or on the other slots.
+// Small problems are bound by launches (ten of them before), large ones by how much of the basis is in flight: a thread
+// keeps its entries of w through subtraction and dots, so no barrier parts the two, and loads kGroup vectors' entries at
+// once, zeros past the last; the dots' sums leave the registers once per group and slice.  50 steps, ten launches / four
+// with a barrier per 256 entries between subtraction and dots / this, ms:  2800 unknowns 3.8 / 2.8 / 2.4, 32640 4.6 / 3.0 /
+// 2.8, 349866 11.4 / 13.2 / 8.4, 1370820 41.4 / 43.6 / 25.7, 32 slots of 32640 31.2 / 28.3 / 23.9, 4 of 349866 30.3 /
+// 33.7 / 27.6.
 namespace {
 // flags, and live / kend / tol of a slot (null for a single space), see GsArgs
 __device__ void givens_column(const GsArgs& a, int b, const cplx* hs, double hk1, cplx* col, cplx* rot, double* rsn) {
@@ -176,11 +180,12 @@ __device__ void givens_column(const GsArgs& a, int b, const cplx* hs, double hk1
 }
 }  // namespace
 
+constexpr int kGroup = 8;
 // MODE 0: hh = V^H w.  1: w -= V hh, c = V^H w.  2: w -= V c, hn = |w|, Hessenberg column and Givens rotation.
 template <int MODE>
 __global__ void __launch_bounds__(kT) k_gs(GsArgs a) {
-    __shared__ cplx hs[kMaxDots], sw[kT], col[kMaxDots], rot[kMaxDots];
-    __shared__ double rsn[kMaxDots], red[kT / 32];
+    __shared__ cplx hs[kMaxDots], col[kMaxDots], rot[kMaxDots];
+    __shared__ double rsn[kMaxDots], red[kT / 32], sums[kT / 32][2 * kGroup];
     __shared__ bool last;
     // the next launch's blocks may take their places; this one's input is the launch before
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -191,66 +196,75 @@ __global__ void __launch_bounds__(kT) k_gs(GsArgs a) {
     cplx* w = a.W + (size_t)b * a.ld;
     if (MODE > 0) {
         const cplx* h = (MODE == 1 ? a.hh : a.c) + (size_t)b * (a.m + 1);
-        for (int i = tid; i < nv; i += kT) hs[i] = h[i];
+        for (int i = tid; i < kMaxDots; i += kT) hs[i] = i < nv ? h[i] : mk(0.0, 0.0);
         __syncthreads();
     }
     const int64_t chunk = (a.n + G - 1) / G, lo = (int64_t)blockIdx.x * chunk, hi = min(a.n, lo + chunk);
-    double sx[kMaxDots / 8], sy[kMaxDots / 8], nrm = 0.0;   // warp q's vectors q, q + 8, ...
+    // kGroup vectors at a time, the ones past the last as zeros: so many loads are always in flight
+    auto group = [&](int i0, int64_t t, cplx (&v)[kGroup]) {
 #pragma unroll
-    for (int e = 0; e < kMaxDots / 8; ++e) sx[e] = sy[e] = 0.0;
-    for (int64_t t0 = lo; t0 < hi; t0 += kT) {
-        const int64_t t = t0 + tid;
-        cplx acc = mk(0, 0);
-        if (t < hi) {
-            acc = w[t];
-            if (MODE > 0) {
-#pragma unroll 8
-                for (int i = 0; i < nv; ++i) acc = acc - hs[i] * V[(size_t)i * a.ldi + t];
-                w[t] = acc;
+        for (int e = 0; e < kGroup; ++e) v[e] = i0 + e < nv ? V[(size_t)(i0 + e) * a.ldi + t] : mk(0.0, 0.0);
+    };
+    if (MODE > 0) {
+        double nrm = 0.0;
+        for (int64_t t = lo + tid; t < hi; t += kT) {
+            cplx acc = w[t];
+            for (int i0 = 0; i0 < nv; i0 += kGroup) {
+                cplx v[kGroup];
+                group(i0, t, v);
+#pragma unroll
+                for (int e = 0; e < kGroup; ++e) acc = acc - hs[i0 + e] * v[e];
             }
+            w[t] = acc;
+            nrm += acc.x * acc.x + acc.y * acc.y;
         }
         if (MODE == 2) {
-            nrm += acc.x * acc.x + acc.y * acc.y;
-        } else {
-            sw[tid] = acc;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+            if (lane == 0) red[q] = nrm;
             __syncthreads();
-#pragma unroll
-            for (int e = 0; e < kMaxDots / 8; ++e) {
-                const int i = q + 8 * e;
-                if (i < nv) {
-                    const cplx* v = V + (size_t)i * a.ldi + t0;
-#pragma unroll
-                    for (int r = lane; r < kT; r += 32)
-                        if (t0 + r < hi) {
-                            const cplx u = v[r], x = sw[r];
-                            sx[e] += u.x * x.x + u.y * x.y;
-                            sy[e] += u.x * x.y - u.y * x.x;
-                        }
-                }
+            if (tid == 0) {
+                double v = 0.0;
+                for (int e = 0; e < kT / 32; ++e) v += red[e];
+                a.npart[(size_t)b * kRedBlocks + blockIdx.x] = v;
             }
-            __syncthreads();
         }
     }
-    if (MODE == 2) {
+    if (MODE < 2) {
+        // a thread has the same entries as above
+        for (int i0 = 0; i0 < nv; i0 += kGroup) {
+            double s[2 * kGroup];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
-        if (lane == 0) red[q] = nrm;
-        __syncthreads();
-        if (tid == 0) {
-            double v = 0.0;
-            for (int e = 0; e < kT / 32; ++e) v += red[e];
-            a.npart[(size_t)b * kRedBlocks + blockIdx.x] = v;
-        }
-    } else {
+            for (int e = 0; e < 2 * kGroup; ++e) s[e] = 0.0;
+            for (int64_t t = lo + tid; t < hi; t += kT) {
+                cplx v[kGroup];
+                group(i0, t, v);
+                const cplx x = w[t];
 #pragma unroll
-        for (int e = 0; e < kMaxDots / 8; ++e) {
-            if (q + 8 * e >= nv) break;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                sx[e] += __shfl_xor_sync(0xffffffffu, sx[e], o);
-                sy[e] += __shfl_xor_sync(0xffffffffu, sy[e], o);
+                for (int e = 0; e < kGroup; ++e) {
+                    s[2 * e] += v[e].x * x.x + v[e].y * x.y;
+                    s[2 * e + 1] += v[e].x * x.y - v[e].y * x.x;
+                }
             }
-            if (lane == 0) a.part[((size_t)b * nv + q + 8 * e) * kRedBlocks + blockIdx.x] = mk(sx[e], sy[e]);
+            // 16 sums over 32 lanes: each step halves the sums a lane carries; lane l ends with sum l / 2
+#pragma unroll
+            for (int o = 16, m = kGroup; o > 1; o >>= 1, m >>= 1)
+#pragma unroll
+                for (int e = 0; e < m; ++e) {
+                    const bool up = (lane & o) != 0;
+                    const double give = up ? s[e] : s[e + m], keep = up ? s[e + m] : s[e];
+                    s[e] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+            __syncthreads();   // the sums of the group before have been read
+            if (!(lane & 1)) sums[q][lane >> 1] = s[0];
+            __syncthreads();
+            if (tid < 2 * kGroup && i0 + tid / 2 < nv) {
+                double v = 0.0;
+#pragma unroll
+                for (int e = 0; e < kT / 32; ++e) v += sums[e][tid];
+                reinterpret_cast<double*>(a.part)[2 * (((size_t)b * nv + i0 + tid / 2) * kRedBlocks + blockIdx.x) + tid % 2] = v;
+            }
         }
     }
     // the last block adds the partial sums
