@@ -193,7 +193,7 @@ struct foggy_handle_s {
     // several right-hand sides in one block (foggy_solve_block, foggy_matvec_block): vectors of
     // nrhs slots, n_unk entries apart
     int blk_nrhs = 0, blk_m = 0;
-    cplx* d_bslab = nullptr;         // operator slabs of bslab_vectors vectors, one per source bucket
+    cplx* d_bslab = nullptr;         // operator slabs of bslab_vectors vectors (kMmaBlock)
     int bslab_vectors = 0;
     cplx* d_bV = nullptr;            // Krylov basis: vector i of slot b at (i nrhs + b) n_unk
     cplx* d_bW = nullptr;            // operator output
@@ -356,6 +356,12 @@ void dfree(foggy_handle h, T*& p) {
         cudaFreeAsync(p, h->stream);
     }
     p = nullptr;
+}
+
+// the block operator's own slabs (apply_operator_block)
+void drop_block_slabs(foggy_handle h) {
+    dfree(h, h->d_bslab);
+    h->bslab_vectors = 0;
 }
 
 #define TRY(x)                      \
@@ -609,13 +615,8 @@ int plan_direct(foggy_handle h) {
     return FOGGY_OK;
 }
 
-// A block's vectors are split as four of them at once would want: by the scene alone, not by how many vectors a launch
-// happens to hold, so that a vector's sums are the same bits whatever else is in the block and however many of its
-// vectors have converged and left.  More CTAs than many vectors need cost their set-up, fewer leave SMs idle when
-// the last few vectors remain; 64 spheres of order 15 get 4 batches a CTA, where one vector wants 3 and 32 want 16.
-// With splits by the count of vectors 32 solves of them took 98.0 ms and 12 applications of 130 spheres 25.8 ms, with
-// these 97.3 and 26.1 (the runs of either differ by 1 and 5 %).
-constexpr int kMmaBlockVectors = 4;
+constexpr size_t kBlockSlabBytes = (size_t)512 << 20;   // slabs of a block's vectors beside the handle's own
+constexpr size_t kVectorSlabBytes = (size_t)16 << 20;   // of one of them
 
 // The tensor-core operator's plan of a use.
 //
@@ -625,8 +626,21 @@ constexpr int kMmaBlockVectors = 4;
 // application, 1000 27.3 -> 24.0 ms, 8 spheres 108 -> 76 us.  The shares' CTAs take about the
 // same number of batches B of four translations, the B that ends first, a CTA costing its batches plus 0.3 of one for
 // its set-up, larger degrees more by their square.  Slabs bound the chunks.
+//
+// A block's B suits 1 to 32 vectors, by the sum of the times over what each count could have: it depends on the scene alone,
+// not on how many vectors a launch happens to hold, so that a vector's sums are the same bits whatever else is in the
+// block and however many of its vectors have converged and left.  With the final sums of many vectors a CTA costs half a batch
+// more.  An application of 2, 5 and 32 vectors with the best B for each count / with this: 64 spheres of order 15 0.148, 0.403,
+// 1.77 / 0.148, 0.309, 1.82 ms, 83 of orders 8..22 0.332, 0.675, 3.73 / 0.325, 0.675, 3.83, 250 of orders 8..28 3.52,
+// 8.46, 51.4 / 3.50, 8.36, 51.4.  More slabs than kVectorSlabBytes for a vector cost more than they spread: they are read
+// again at the end, and fewer vectors go at once (83 lognormal spheres, 5 vectors: 1.22 ms without the bound, 0.97).
 int make_mma_plan(foggy_handle h, MmaUse u, bool sum, MmaPlan& p) {
-    const int nb = h->nbuckets, nv = u == kMmaBlock ? kMmaBlockVectors : 1, per = u == kMmaStatic ? 1 : h->cmax;
+    const int nb = h->nbuckets;
+    int per = u == kMmaStatic ? 1 : h->cmax;
+    if (u == kMmaBlock)
+        per = (int)std::max<size_t>(1, std::min<size_t>(per, kVectorSlabBytes / ((size_t)nb * h->n_unk * sizeof(cplx))));
+    const std::vector<int> counts = u == kMmaBlock ? std::vector<int>{1, 2, 4, 8, 16, 32} : std::vector<int>{1};
+    const double setup = u == kMmaBlock ? 0.5 : 0.3;
     p.use.nb = nb;
     std::vector<MmaWork> work;
     for (int cls = 4; cls >= 0; --cls) {
@@ -642,24 +656,32 @@ int make_mma_plan(foggy_handle h, MmaUse u, bool sum, MmaPlan& p) {
             const int batches = (h->launches_direct[i].nsources + 3) / 4;
             return std::max(1, std::min({per, batches, (batches + B - 1) / B}));
         };
-        double best = 1e300;
-        int bestB = 1;
-        for (int B : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 128}) {
+        auto time_of = [&](int B, int nv) {
             double total = 0.0, longest = 0.0;
             int64_t ctas = 0;
             for (int i : in) {
                 const DirectBucket& b = h->launches_direct[i];
                 const int batches = (b.nsources + 3) / 4, c = chunks_for(i, B);
-                const double cost = ((batches + c - 1) / c + 0.3) * (double)b.pp * b.pp;
+                const double cost = ((batches + c - 1) / c + setup) * (double)b.pp * b.pp;
                 const int64_t n = (int64_t)b.ntargets * nv * c;
                 total += cost * n;
                 ctas += n;
                 longest = std::max(longest, cost);
             }
             // equal CTAs run in waves; unequal ones, the largest first, leave half of one at the end
-            const double t = in.size() == 1 ? std::ceil((double)ctas / slots) * longest
-                             : ctas <= slots ? longest
-                                             : total / slots + 0.5 * longest;
+            return in.size() == 1 ? std::ceil((double)ctas / slots) * longest
+                   : ctas <= slots ? longest
+                                   : total / slots + 0.5 * longest;
+        };
+        const std::initializer_list<int> sizes = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 128};
+        std::vector<double> least(counts.size(), 1e300);
+        for (int B : sizes)
+            for (size_t v = 0; v < counts.size(); ++v) least[v] = std::min(least[v], time_of(B, counts[v]));
+        double best = 1e300;
+        int bestB = 1;
+        for (int B : sizes) {
+            double t = 0.0;
+            for (size_t v = 0; v < counts.size(); ++v) t += time_of(B, counts[v]) / least[v];
             if (t < best * 0.999) {
                 best = t;
                 bestB = B;
@@ -1561,8 +1583,7 @@ void free_scene(foggy_handle h) {
     dfree(h, h->d_b);
     dfree(h, h->d_pq);
     dfree(h, h->d_partial);
-    dfree(h, h->d_bslab);
-    h->bslab_vectors = 0;
+    drop_block_slabs(h);
     free_mma_plans(h);
     dfree(h, h->d_stab);
     dfree(h, h->d_stab32);
@@ -2840,7 +2861,6 @@ namespace {
 // Tile width R per launch shape, chosen by timing: (FP32, pair tables, largest degree, log2 of the
 // target count, block width up to 8) -> R.  Process-wide, as the choice depends on the shape only.
 constexpr size_t kBlockKeepBytes = (size_t)256 << 20;   // host vectors of foggy_matvec_block kept on the device
-constexpr size_t kBlockSlabBytes = (size_t)128 << 20;   // slabs of many vectors at once on the tensor cores
 std::mutex g_tile_mu;
 std::map<std::tuple<int, int, int, int, int>, int> g_tile_cache;
 
@@ -2953,7 +2973,7 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
         // coaxial block comes from L2 after the first.  83 spheres, 5 right-hand sides to 1e-6: 161 -> 55 ms a request
         // (the tile autotuner's runs are gone too).  As many vectors at a time as have slabs: the handle's own, or a
         // buffer of up to kBlockSlabBytes where that holds more, so that the waves of a small scene's CTAs end
-        // together (64 spheres, 32 vectors: 14 + 14 + 4 vectors took 9 waves of 296 CTAs, 32 take 7).
+        // together (83 lognormal spheres, 32 vectors: 5.89 ms in groups of 8, 5.57 at once).
         Trace tr("block operator (FP64)");
         DirectArgs a = ba.d;
         const SlabUse& use = h->mma_plans[kMmaBlock][0].use;
@@ -2965,7 +2985,7 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
         const int fit = (int)std::min<size_t>(nrhs, std::min(kBlockSlabBytes, room / 4) / (one * sizeof(cplx)));
         if (nrhs > most && fit > most) {
             if (h->bslab_vectors < fit) {
-                dfree(h, h->d_bslab);
+                drop_block_slabs(h);
                 h->bslab_vectors = dalloc(h, &h->d_bslab, one * fit) == FOGGY_OK ? fit : 0;
             }
             if (h->bslab_vectors > most) {
