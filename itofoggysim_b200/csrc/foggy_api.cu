@@ -316,10 +316,13 @@ void pinned_release(char* q) {
     P.free.push_back(q);
 }
 
+void drop_block_slabs(foggy_handle h);
+
 template <class T>
 int dalloc(foggy_handle h, T** p, size_t count) {
     size_t bytes = count * sizeof(T);
     if (bytes == 0) bytes = 16;
+    if (h->budget && h->bytes_in_use + bytes > h->budget) drop_block_slabs(h);
     if (h->budget && h->bytes_in_use + bytes > h->budget)
         return fail(h, FOGGY_ERR_NOMEM, "device memory budget exceeded (" + std::to_string(h->bytes_in_use + bytes) +
                                             " > " + std::to_string(h->budget) + " bytes)");
@@ -358,10 +361,18 @@ void dfree(foggy_handle h, T*& p) {
     p = nullptr;
 }
 
-// the block operator's own slabs (apply_operator_block)
+// The block operator's own slabs (apply_operator_block) give way to whatever else needs the budget; their uses lie
+// before the free on the handle's stream.
 void drop_block_slabs(foggy_handle h) {
     dfree(h, h->d_bslab);
     h->bslab_vectors = 0;
+}
+
+// what the budget leaves, those slabs counted as free
+size_t budget_room(foggy_handle h) {
+    const auto it = h->alloc_bytes.find(h->d_bslab);
+    const size_t used = h->bytes_in_use - (h->d_bslab && it != h->alloc_bytes.end() ? it->second : 0);
+    return h->budget > used ? h->budget - used : 0;
 }
 
 #define TRY(x)                      \
@@ -881,7 +892,7 @@ int ensure_pair_tables(foggy_handle h, bool fp32 = false) {
     const size_t offb = h->d_pair_off ? 0 : (size_t)npairs * 2 * sizeof(int64_t);
     const size_t b64 = h->d_stab ? 0 : (size_t)tot * sizeof(cplx);
     const size_t b32 = h->d_stab32 ? 0 : (size_t)tot * sizeof(cplxf);
-    const size_t room = h->budget > h->bytes_in_use ? h->budget - h->bytes_in_use : 0;
+    const size_t room = budget_room(h);
     const size_t reserve = (size_t)(h->prm.gmres_restart + 4) * (size_t)h->n_unk * sizeof(cplx) + ((size_t)4 << 30);
     const bool force = h->prm.pair_tables == 1;
     const bool fits64 = force || offb + b64 + reserve <= room;
@@ -1310,7 +1321,7 @@ int ensure_fmm_tables(foggy_handle h, const TransArgs& base, const std::vector<F
     }
     const bool mixed = h->prm.precision == 1;
     const size_t need = (size_t)entries * (sizeof(cplx) + (mixed ? sizeof(cplxf) : 0)) + (size_t)total * sizeof(int64_t);
-    const size_t room = h->budget > h->bytes_in_use ? h->budget - h->bytes_in_use : 0;
+    const size_t room = budget_room(h);
     const size_t reserve = (size_t)(h->prm.gmres_restart + 4) * (size_t)h->n_unk * sizeof(cplx) + ((size_t)1 << 30);
     if (h->prm.pair_tables == 0 && need + reserve > room) {
         h->fmm_tab_ready = true;   // do not fit: the passes sum S from the Gaunt table
@@ -2980,9 +2991,7 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
         int most = std::max(1, h->nbuckets * h->cmax / std::max(1, use.per_rhs));
         const size_t one = (size_t)use.per_rhs * h->n_unk;
         // at most a quarter of what the budget leaves: a tight one is for the calls to come
-        const size_t room = (h->budget > h->bytes_in_use ? h->budget - h->bytes_in_use : 0) +
-                            (size_t)h->bslab_vectors * one * sizeof(cplx);
-        const int fit = (int)std::min<size_t>(nrhs, std::min(kBlockSlabBytes, room / 4) / (one * sizeof(cplx)));
+        const int fit = (int)std::min<size_t>(nrhs, std::min(kBlockSlabBytes, budget_room(h) / 4) / (one * sizeof(cplx)));
         if (nrhs > most && fit > most) {
             if (h->bslab_vectors < fit) {
                 drop_block_slabs(h);

@@ -69,3 +69,31 @@ def test_solve(native, tables):
         y = s.solve_block(x0=np.zeros_like(x[:2]))[0]
     assert np.array_equal(fresh[[0, 5]], alone[[0, 5]])
     assert np.array_equal(fresh[:2], y)
+
+
+def test_slabs_give_way(native):
+    """A block application keeps slabs for its vectors in what the budget leaves; a solve that needs that memory afterwards
+    gets it: the budgets at which a block solve succeeds are the same with and without an application before."""
+    from itofoggysim_b200 import _native, solver
+    n = 16
+    rng = np.random.default_rng(3)
+    sc = dataclasses.replace(scene([6] * 90, 3, 21), wave_theta=rng.uniform(0.1, 3.0, n), wave_phi=rng.uniform(0, 6, n),
+                             jones=np.tile([1.0, 0.0, 0.0, 0.0], (n, 1)), wave_g=np.ones(n), wave_phase=np.zeros(n),
+                             wave_d0=np.zeros((n, 3)), gmres_restart=60, gmres_tolerance=1e-3)
+    X = vectors(sc, 60)
+
+    def solved(budget, before):
+        try:
+            with solver.MultiSphereSolver(sc, pair_tables=1, memory_budget=budget) as s:
+                if before:
+                    s.calculate_vector_b_block(X)
+                s.solve_block()
+            return True
+        except _native.FoggyError as e:
+            assert e.code == _native.FOGGY_ERR_NOMEM
+            return False
+
+    budgets = [mb << 20 for mb in range(40, 400, 12)]
+    alone = [solved(b, False) for b in budgets]
+    assert True in alone and False in alone
+    assert alone == [solved(b, True) for b in budgets]
