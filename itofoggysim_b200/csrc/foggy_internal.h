@@ -32,6 +32,8 @@ void build_delta_table(int pmax, std::vector<double>& out);
 // ceiling is a process-wide attribute of the function: handles launching the same kernel from
 // several threads only ever raise it, under one lock, so no launch finds it lowered by another.
 void raise_smem_ceiling(const void* func, size_t bytes);
+// largest order of the FP64 operator on the tensor cores (k_direct_mma.cu)
+constexpr int kMmaDegree = 31;
 // device bytes a direct solve will hold; pair tables counted when pair_tables == 1 (their size in
 // *table_bytes either way)
 int64_t estimate_solve_bytes(const foggy_params& prm, int N, const int* param_index, int NP, const int* n_range,

@@ -134,7 +134,6 @@ size_t translation_pair_smem_bytes(int pmax);
 void launch_direct(const DirectArgs& a, const DirectBucket& b, cudaStream_t s);
 
 // k_direct_mma.cu -- the FP64 operator on the tensor cores, for orders up to kMmaDegree over the pair tables
-constexpr int kMmaDegree = 31;
 struct MmaTabs {
     const double* frag;        // d^n(pi/2) as fragments, degree by degree (build_mma_tables)
     const double2* wf;         // factors of the coaxial step's w, one entry per (order, degree)

@@ -205,9 +205,14 @@ int32_t foggy_server_submit(foggy_server S, const foggy_request* q, int64_t* id)
     r->g = copy_of(q->g, (size_t)q->nw);
     r->phase = copy_of(q->phase, (size_t)q->nw);
     r->d0 = copy_of(q->d_0_i, 3 * (size_t)q->nw);
-    // pair tables when they take at most an equal share of the budget beside the solve itself
+    // pair tables when they take at most an equal share of the budget beside the solve itself; a mixed-precision solve
+    // of the orders that the FP64 tensor-core operator takes builds the double-precision ones alone
     int64_t tb = 0;
-    const int64_t base = foggy::estimate_solve_bytes(r->prm, r->N, r->pidx.data(), r->NP, r->nr.data(), 0, &tb);
+    int top = 0;
+    for (int j = 0; j < r->N; ++j) top = std::max(top, std::min(r->nr[2 * r->pidx[j] + 1], r->prm.n_range[1]));
+    foggy_params need = r->prm;
+    if (need.precision == 1 && top <= foggy::kMmaDegree) need.precision = 0;
+    const int64_t base = foggy::estimate_solve_bytes(need, r->N, r->pidx.data(), r->NP, r->nr.data(), 0, &tb);
     const int share = (int)std::max<size_t>(1, S->workers.size());
     bool tables = r->prm.pair_tables == 1 || (r->prm.pair_tables == 0 && base + tb <= S->budget / share);
     r->prm.pair_tables = tables ? 1 : -1;
