@@ -3268,10 +3268,10 @@ int32_t foggy_matvec_block(foggy_handle h, int32_t nrhs, int32_t precision, cons
         dfree(h, X);
         return rc;
     };
-    // the identity rows above a sphere's degree come from x: vectors from the host are kept while the pool gives room,
-    // else copied again
+    // the identity rows above a sphere's degree come from x: vectors from the host are kept where they take at most a
+    // quarter of what the budget leaves, and the pool gives room, else copied again
     cplx* kept = nullptr;
-    if (mem == FOGGY_MEM_HOST && (size_t)nrhs * len * sizeof(cplx) <= kBlockKeepBytes &&
+    if (mem == FOGGY_MEM_HOST && (size_t)nrhs * len * sizeof(cplx) <= std::min(kBlockKeepBytes, budget_room(h) / 4) &&
         talloc(h, &kept, (size_t)nrhs * len * sizeof(cplx)) != cudaSuccess) {
         cudaGetLastError();
         kept = nullptr;
