@@ -2470,6 +2470,8 @@ int64_t estimate_solve_bytes(const foggy_params& prm, int N, const int* param_in
     return bytes + (pair_tables == 1 ? tb : 0);
 }
 
+// integers of a block solve's slot: live, kend, flags, ticket
+constexpr int kBlockInts = 4;
 int64_t estimate_block_bytes(const foggy_params& prm, int N, const int* param_index, int NP, const int* n_range,
                              int nrhs) {
     const int pg = prm.n_range[1];
@@ -2479,7 +2481,8 @@ int64_t estimate_block_bytes(const foggy_params& prm, int N, const int* param_in
         n_unk += 2 * (int64_t)p * (p + 2);
     }
     const int64_t m = prm.gmres_restart, v = (int64_t)sizeof(cplx);
-    return (m + 5) * nrhs * n_unk * v + nrhs * ((m + 1) * (m + 5 + kRedBlocks) * v + (m + 5 + kRedBlocks) * 8 + 12);
+    return (m + 5) * nrhs * n_unk * v + nrhs * ((m + 1) * (m + 5 + kRedBlocks) * v + (m + 5 + kRedBlocks) * 8 +
+                                                kBlockInts * (int64_t)sizeof(int));
 }
 }  // namespace foggy
 
@@ -3038,8 +3041,8 @@ int ensure_block_ws(foggy_handle h, int nrhs, int m) {
     TRY(dalloc(h, &h->d_bsmall, nb * ((size_t)(m + 1) * m + m + 4 * (size_t)(m + 1) + (size_t)(m + 1) * kRedBlocks)));
     // sn m, bnorm, beta, hn, tol, res per slot; norm partials kRedBlocks per slot
     TRY(dalloc(h, &h->d_breal, nb * ((size_t)m + 5 + kRedBlocks)));
-    TRY(dalloc(h, &h->d_bint, 4 * nb));
-    CK(h, cudaMemsetAsync(h->d_bint, 0, 4 * nb * sizeof(int), h->stream));
+    TRY(dalloc(h, &h->d_bint, kBlockInts * nb));
+    CK(h, cudaMemsetAsync(h->d_bint, 0, kBlockInts * nb * sizeof(int), h->stream));
     h->blk_nrhs = nrhs;
     h->blk_m = m;
     return FOGGY_OK;
