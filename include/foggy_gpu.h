@@ -98,8 +98,10 @@ typedef struct foggy_params {
                                     at every restart in FP64, so the restarts refine to
                                     gmres_tolerance.  foggy_matvec stays FP64.  Where the
                                     FP64 operator runs on the tensor cores (orders up to 31;
-                                    blocks: with pair tables) it is as fast, and the Arnoldi steps of
-                                    the direct operator use it instead                      */
+                                    blocks: with pair tables) it is as fast, and the Arnoldi
+                                    steps of the direct operator use it instead; so do those
+                                    ML-FMM passes that run there (M2L and near field of 4096
+                                    and more list entries over cached blocks)               */
 } foggy_params;
 
 /* Per-solve statistics (the reference prints these; here they are returned). */
