@@ -535,7 +535,7 @@ MmaTabs mma_tabs(foggy_handle h) {
 // Whether the FP64 operator runs on the tensor cores: orders up to kMmaDegree, with the pair tables or without.  It is
 // the faster one at every order it takes (222 spheres of one order over tables: 7 0.29 against 1.39 ms, 15 0.75 / 2.0,
 // 23 1.8 / 4.9, 31 3.4 / 9.7; 211 spheres of orders 5..9 that sum S: 3.8 / 6.5).
-bool mma_operator(foggy_handle h, const DirectArgs&) { return h->pmax <= kMmaDegree; }
+bool mma_operator(foggy_handle h) { return h->pmax <= kMmaDegree; }
 
 DirectArgs direct_args(foggy_handle h, const cplx* x) {
     DirectArgs a;
@@ -618,8 +618,9 @@ int plan_direct(foggy_handle h) {
             b.pp = std::max(bp[t], bp[s]);
             h->launches_direct.push_back(b);
         }
-    // made here, so that no later call allocates for them
+    // made here, so that no later call allocates for them; a scene of an order above has none
     free_mma_plans(h);
+    if (!mma_operator(h)) return FOGGY_OK;
     for (int u = 0; u < kMmaUses; ++u)
         for (int sum = 0; sum < (u == kMmaBlock ? 1 : 2); ++sum)   // blocks without tables run on the CUDA cores
             TRY(make_mma_plan(h, (MmaUse)u, sum != 0, h->mma_plans[u][sum]));
@@ -657,7 +658,7 @@ int make_mma_plan(foggy_handle h, MmaUse u, bool sum, MmaPlan& p) {
     for (int cls = 4; cls >= 0; --cls) {
         std::vector<int> in;
         for (int i = 0; i < nb * nb; ++i)
-            if (h->launches_direct[i].pp <= kMmaDegree && mma_class(h->launches_direct[i].pp, sum) == cls) in.push_back(i);
+            if (mma_class(h->launches_direct[i].pp, sum) == cls) in.push_back(i);
         if (in.empty()) continue;
         std::stable_sort(in.begin(), in.end(),
                          [&](int a, int b) { return h->launches_direct[a].pp > h->launches_direct[b].pp; });
@@ -1511,7 +1512,7 @@ int apply_operator(foggy_handle h, const cplx* x, cplx* y, bool fp32 = false) {
     DirectArgs a = direct_args(h, x);
     // also for the Arnoldi steps of a mixed-precision solve, unless the single-precision tables alone fit: reading those
     // beats summing S in FP64
-    const bool mma = mma_operator(h, a) && !(fp32 && h->stab32_ready && !h->stab_ready);
+    const bool mma = mma_operator(h) && !(fp32 && h->stab32_ready && !h->stab_ready);
     a.fp32 = (!mma && fp32 && h->stab32_ready) ? 1 : 0;
     Trace tr(a.fp32 ? "operator (FP32)" : "operator (FP64)");
     if (mma) {
@@ -2212,7 +2213,7 @@ int32_t foggy_matvec(foggy_handle h, const double* x, double* y, int32_t mem) {
     if (h->prm.matvec_mode == FOGGY_MATVEC_DIRECT) {
         TRY(ensure_pair_tables(h));
         const DirectArgs a = direct_args(h, h->d_tmp_in);
-        packed = mma_operator(h, a);
+        packed = mma_operator(h);
         Trace tr("operator (FP64)");
         if (packed) TRY(launch_mma(h, a, kMmaSingle, 1, h->d_tmp_in, yr, xr));
     }
@@ -2842,7 +2843,7 @@ extern "C" int32_t foggy_matvec_static(foggy_handle h, const double* x, double* 
     DirectArgs a = direct_args(h, xin);
     a.partial = partial;
     a.cmax = 1;
-    if (mma_operator(h, a)) {
+    if (mma_operator(h)) {
         TRY(launch_mma(h, a, kMmaStatic, 1, xin, yout));
     } else {
         for (const DirectBucket& b : h->launches_direct) {
@@ -2982,7 +2983,7 @@ int apply_operator_block(foggy_handle h, const cplx* X, cplx* Y, int nrhs, bool 
     const BlockArgs ba = block_args(h, X, Y, nrhs, fp32);
     // without tables the CUDA-core kernel sums S once for a tile of vectors (for one too: a block's last vector keeps the
     // operator that it had beside the others)
-    if (!must32 && mma_operator(h, ba.d) && ba.d.pt.stab) {
+    if (!must32 && mma_operator(h) && ba.d.pt.stab) {
         // One vector per CTA: a batch's set-up that vectors could share is small beside its products, and the pair's
         // coaxial block comes from L2 after the first.  83 spheres, 5 right-hand sides to 1e-6: 161 -> 55 ms a request
         // (the tile autotuner's runs are gone too).  As many vectors at a time as have slabs: the handle's own, or a
@@ -3448,7 +3449,7 @@ int32_t foggy_block_tiles(foggy_handle h, int32_t precision, int32_t nrhs, int32
         const DirectBucket& b = h->launches_direct[i];
         int R = 0;
         // one vector per CTA on the tensor cores
-        if (!ba.d.fp32 && mma_operator(h, ba.d) && tabs) R = 1;
+        if (!ba.d.fp32 && mma_operator(h) && tabs) R = 1;
         else rc = choose_tile(h, ba, b, tabs, &R);
         out[4 * i] = b.ntargets;
         out[4 * i + 1] = b.nsources;
