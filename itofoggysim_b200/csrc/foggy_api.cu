@@ -999,8 +999,10 @@ void free_fmm(foggy_handle h) {
 // few boxes still fill the GPU; their partial sums need fewer than 2 kFmmFill slabs of one target.
 constexpr int kFmmFill = 148 * 6;
 constexpr int kFmmChunks = 16;
-// list entries from which a pass runs on the tensor cores: below, its time is a launch or two either way.  500 long-wave
-// spheres, per application: near field 318 -> 93 us; M2L (levels of orders 17 and 11) 855 -> 350 us.
+// List entries from which a pass runs on the tensor cores.  Below, passes over cached blocks keep the bits of those that
+// sum S; they would be faster there too.  An application with every pass of lists of four and more on them / with none: 500
+// long-wave spheres (23192 and 9786 entries of M2L and near field) 389 / 1021 us, 300 (3004, 21452) 227 / 767, 150 (2450,
+// 5340) 126 / 278, 64 (1384, 976) 82 / 123; with this line 389, 302, 167 and 123.
 constexpr int kFmmMmaEntries = 4096;
 
 // Expansion order of the boxes of level l.  The reference expands every box to its global order
