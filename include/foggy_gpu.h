@@ -246,8 +246,9 @@ int32_t foggy_universal_index(int32_t n, const double* points, int32_t l, int64_
 /* Device bytes a direct-operator solve of this scene holds at its peak, from the plan the handle
  * follows (scene arrays, operator slabs, Krylov workspace, staging, order tables), into
  * solve_bytes, and the pair tables' bytes into table_bytes (FP64, plus FP32 when
- * params->precision = 1).  The solve server admits requests by these.  Host only: no handle, no
- * GPU. */
+ * params->precision = 1: the most such a handle builds; up to order 31 it does so only where FP32 is
+ * asked for by name or FP64 does not fit, so the solve server, which admits requests by these bytes,
+ * counts the FP64 tables alone for them).  Host only: no handle, no GPU. */
 int32_t foggy_estimate_solve_bytes(const foggy_params* params, int32_t n_spheres, const int32_t* param_index,
                                    int32_t n_param, const int32_t* n_range, int64_t* solve_bytes,
                                    int64_t* table_bytes);
