@@ -1,5 +1,5 @@
 """The oracle's Wigner 3j symbols against Racah's sum in exact rational arithmetic, and the time of the translation
-blocks that are made of them: the oracle serves as the judge of every operator, up to order 45.
+blocks that are made of them: every operator is tested against the oracle, up to order 45.
 
 The recurrence carries 64 bits of mantissa over at most 2 min(j1, j2) + 1 <= 200 steps from either end, a few roundings
 each, so its error is some 1e-17 of the family's largest value; with the rounding to 53 bits that is 2e-16 of a symbol
